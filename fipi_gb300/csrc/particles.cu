@@ -5,11 +5,11 @@
 //    (cluster.cpp:140-165), a stable LSD radix sort of (key, particle id) and
 //    offsets by binary search; ids inside a cell are ascending, which is the
 //    order the reference's linked lists hold them in (linked_list.cpp:30-43);
-//  - contact forces one warp per home cell (cluster.cpp:174-275): each lane
-//    owns one particle of the cell and walks the 27 neighbour cells in the
-//    reference's (k, j, i) order; every pair is evaluated from the lower id's
-//    side exactly as the reference does and the result is applied with the
-//    reference's sign, so forces are deterministic and atomic-free;
+//  - contact forces (cluster.cpp:174-275) gathered per particle over the 27
+//    neighbour cells with the reference's sign rule, summed in a fixed
+//    order: deterministic and atomic-free (k_f_pp_warp, k_f_pp_fast; k_f_pp,
+//    one warp per home cell in the reference's order, for the cell grids
+//    they do not take and for the pair lists);
 //  - interpolation, attachment force, Heun advection and periodic wrap per
 //    particle (field.cpp:223-248, element.cpp:55-185);
 //  - spreading (cluster.cpp:344-410) as a sorted segmented reduction: the
@@ -57,7 +57,10 @@ struct PC {
     double inv_dc[3];  // 1/d_cell
     double mdc[3];     // margin/d_cell
     double drag;       // 6 pi mu: the Stokes drag is drag * r
-    float f_req, f_req2, f_kn, f_dc[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
+    double img[3];     // d_cell (n_cell - 2): the minimum-image threshold
+    double inv_req2;    // 1/r_eq^2
+    double to_unit[3];  // 2^32 / L: positions as 32-bit fractions of the box
+    float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_unit[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
 };
 
 static PC make_pc(const fipi_ctx* ctx) {
@@ -94,10 +97,22 @@ static PC make_pc(const fipi_ctx* ctx) {
         c.inv_dc[a] = 1.0 / c.dc[a];
         c.mdc[a] = c.margin / c.dc[a];
         c.f_dc[a] = (float)c.dc[a];
+        c.img[a] = c.dc[a] * (c.nc[a] - 2);
+        c.to_unit[a] = 4294967296.0 / c.L[a];
+        c.f_unit[a] = (float)(c.L[a] / 4294967296.0);
     }
     c.drag = 6.0 * c.pi * c.mu;
     c.f_req = (float)c.r_eq;
     c.f_req2 = c.f_req * c.f_req;
+    c.inv_req2 = 1.0 / (c.r_eq * c.r_eq);
+    // FP32 selection radius: a separation formed from cell-relative FP32
+    // coordinates of up to 2 d_cell is off by less than 16 * 2^-24 d_cell per
+    // axis (two conversions, the offset and its product, two subtractions)
+    {
+        const double dcm = std::max(c.dc[0], std::max(c.dc[1], c.dc[2]));
+        const double rs = c.r_eq + 32.0 * dcm / 16777216.0;
+        c.f_req2_sel = (float)(rs * rs * (1.0 + 1e-6));
+    }
     c.f_kn = (float)c.k_n;
     c.f_inv_vol = (float)(1.0 / (c.dx * c.dy * c.dz));
     c.f_tanh2 = (float)c.tanh2;
@@ -347,12 +362,27 @@ __global__ void k_cells_place(PC pc, const double* __restrict__ p, const unsigne
     }
 }
 
+// What the contact forces (k_f_pp_warp) read of particle i at sorted position
+// s: its position relative to its cell in FP32 with the id and, with ipos
+// (mixed form, by id), as 32-bit fractions of the box (2^32 wraps to 0, as
+// the box does).
+__device__ __forceinline__ void sorted_pos(const PC& pc, const double* __restrict__ p, int i, int cx, int cy, int cz,
+                                           int s, float4* spos, int4* ipos) {
+    const int n = pc.n;
+    const double x = p[i], y = p[n + i], z = p[2 * n + i];
+    spos[s] = make_float4((float)fma((double)-cx, pc.dc[0], x), (float)fma((double)-cy, pc.dc[1], y),
+                          (float)fma((double)-cz, pc.dc[2], z), __int_as_float(i));
+    if (ipos)
+        ipos[i] = make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(x * pc.to_unit[0]),
+                            (int)(unsigned)(unsigned long long)__double2ll_rn(y * pc.to_unit[1]),
+                            (int)(unsigned)(unsigned long long)__double2ll_rn(z * pc.to_unit[2]), 0);
+}
+
 // One warp per cell: rank of each id among the cell's ids.  With spos the
-// sorted cell-relative FP32 positions of the mixed-form contact forces are
-// written as well (what k_sorted_pos computes).
+// sorted positions of the contact forces are written as well.
 __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __restrict__ off, int ncells,
                               const unsigned* __restrict__ tmp, unsigned* ids, unsigned* skeys,
-                              unsigned long long* ymax, int* it_mark, float4* spos) {
+                              unsigned long long* ymax, int* it_mark, float4* spos, int4* ipos) {
     const int cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (ymax && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -363,26 +393,18 @@ __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __
     if (cell >= ncells) return;
     const int beg = off[cell], end = off[cell + 1];
     const int cx = cell % pc.nc[0], cy = (cell / pc.nc[0]) % pc.nc[1], cz = cell / (pc.nc[0] * pc.nc[1]);
-    const int n = pc.n;
     for (int e = beg + lane; e < end; e += 32) {
         const unsigned id = tmp[e];
         int r = 0;
         for (int j = beg; j < end; ++j) r += tmp[j] < id;
         ids[beg + r] = id;
         skeys[beg + r] = (unsigned)cell;
-        if (spos) {  // mixed form only: one fused multiply-add per axis
-            float4 v;
-            v.x = (float)fma((double)-cx, pc.dc[0], p[id]);
-            v.y = (float)fma((double)-cy, pc.dc[1], p[n + id]);
-            v.z = (float)fma((double)-cz, pc.dc[2], p[2 * n + id]);
-            v.w = __int_as_float((int)id);
-            spos[beg + r] = v;
-        }
+        if (spos) sorted_pos(pc, p, (int)id, cx, cy, cz, beg + r, spos, ipos);
     }
 }
 
 // Returns true when it also computed it_mark (asked for by `want_it_mark`).
-// With spos the sorted FP32 positions of the mixed-form contact forces too;
+// With spos the sorted FP32 positions of the contact forces too;
 // `fast` takes the mixed form's cell keys (cell_key<true>).
 static bool build_cells(fipi_ctx* ctx, const double* p_dev, bool want_it_mark = false, float4* spos = nullptr,
                         bool fast = false) {
@@ -401,7 +423,7 @@ static bool build_cells(fipi_ctx* ctx, const double* p_dev, bool want_it_mark = 
     }
     { LaunchScope ls_(ctx, "cell offsets", 0.0); k_cells_scan<<<1, 1024, 0, ctx->stream>>>(b.cell_cnt, b.ncells, b.cell_off); }
     { LaunchScope ls_(ctx, "cell placement", 0.0); k_cells_place<<<nb, kPT, 0, ctx->stream>>>(pc, p_dev, b.keys_alt, b.ids_alt, b.cell_off, b.keys, ym); }
-    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos); }
+    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos, b.ipos); }
     std::swap(b.keys, b.keys_alt);  // sorted keys now in keys
     return want_it_mark;
 }
@@ -535,33 +557,26 @@ __global__ void k_f_pp(PC pc, const double* __restrict__ p, const unsigned* __re
     }
 }
 
+// k_cells_order's sorted positions, for callers that built the list without them.
+__global__ void k_sorted_pos(PC pc, const double* __restrict__ p, const unsigned* __restrict__ keys,
+                             const unsigned* __restrict__ ids, float4* __restrict__ spos, int4* __restrict__ ipos) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= pc.n) return;
+    const unsigned key = keys[s];
+    sorted_pos(pc, p, (int)ids[s], key % pc.nc[0], (key / pc.nc[0]) % pc.nc[1], key / (pc.nc[0] * pc.nc[1]), s, spos,
+               ipos);
+}
+
 // Mixed-form contact forces when every axis has at least 4 cells.  Then
 // the reference's minimum-image rule (shift d by L when |d| exceeds
 // d_cell (n_cell - 2), cluster.cpp:225-232) shifts exactly the pairs whose
 // neighbour cell was reached through the periodic wrap, so d can be formed
 // from cell-relative FP32 coordinates plus the neighbour cell's offset
-// (di, dj, dk) d_cell, with no per-pair test.  A warp owns a home cell;
-// candidates are read 32 at a time (coalesced float4: x, y, z relative to
-// their cell, id) and broadcast by shuffles.  The force on the home
+// (di, dj, dk) d_cell, with no per-pair test.  The force on the home
 // particle from a pair is (d/|d|) s with d = p_i - p_j for either id
 // order (exactly the reference's sign rule), summed in the reference's
 // cell order.
-__global__ void k_sorted_pos(PC pc, const double* __restrict__ p, const unsigned* __restrict__ keys,
-                             const unsigned* __restrict__ ids, float4* __restrict__ spos) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= pc.n) return;
-    const unsigned key = keys[s];
-    const int i = (int)ids[s];
-    const int cx = key % pc.nc[0], cy = (key / pc.nc[0]) % pc.nc[1], cz = key / (pc.nc[0] * pc.nc[1]);
-    const int n = pc.n;
-    float4 v;
-    v.x = (float)(p[i] - cx * pc.dc[0]);
-    v.y = (float)(p[n + i] - cy * pc.dc[1]);
-    v.z = (float)(p[2 * n + i] - cz * pc.dc[2]);
-    v.w = __int_as_float(i);
-    spos[s] = v;
-}
-
+//
 // One block per home cell, one warp per (dk, dj) neighbour row of three
 // cells (9 warps); the nine partial forces of each home particle are then
 // added in the reference's (k, j) cell order, so the result is
@@ -702,6 +717,276 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
         }
         __syncthreads();
     }
+}
+
+// Contact forces, one block per home cell (or per share of its particles),
+// one warp per home particle: the FP64 form, and the mixed form with 3
+// cells on an axis.
+//
+// The block stages the candidates of the 27 neighbour cells in shared memory
+// in the reference's cell order, as FP32 positions in the home cell's frame
+// (cell-relative coordinates plus the neighbour cell's offset (di, dj, dk)
+// d_cell).  About one candidate in twelve lies within r_eq (4/3 pi r_eq^3
+// against 27 cells), so these separations only select: candidates within
+// r_eq plus their rounding bound (f_req2_sel) are queued by ballot, and every
+// 32 of them are evaluated with all lanes busy.  The evaluation takes the
+// minimum image of cluster.cpp:225-232 (shift d by L when |d| exceeds
+// d_cell (n_cell - 2)):
+//  FP64 form   the rule itself on the FP64 positions (FP64 issues at 1/64 of
+//              the FP32 rate: 40 pairs a particle instead of 500);
+//  mixed form  positions as 32-bit fractions of the box, whose wrapping
+//              difference is the nearest image: exact to L 2^-32 (FP32 cell
+//              coordinates: d_cell 2^-23), then FP32.
+// Both select and evaluate the same image as the rule for every pair that
+// can interact: with at least 4 cells per axis the rule shifts exactly the
+// pairs reached through the periodic wrap, and with 3 it differs only for
+// pairs further apart than d_cell; f_pp_path asks for r_eq <= d_cell
+// there, and for r_eq < L / 2.  Lane sums meet in a fixed shuffle order:
+// deterministic.
+constexpr int kFppWarps = 4;
+constexpr int kFppStage = 768;  // staged candidates (12 KB); more go in several rounds
+
+struct FppShared {
+    float4 cand[kFppStage];  // x, y, z in the home cell's frame, id
+    int queue[kFppWarps][64];
+    int beg[27], pre[28];  // start and exclusive count prefix of the neighbour cells
+};
+
+// Starts and prefix counts of the 27 neighbour cells (first warp).
+__device__ __forceinline__ void fpp_cells(const PC& pc, int cell, const int* __restrict__ off, FppShared& sh) {
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    const int ci = cell % pc.nc[0], cj = (cell / pc.nc[0]) % pc.nc[1], ck = cell / (pc.nc[0] * pc.nc[1]);
+    int beg = 0, cnt = 0;
+    if (lane < 27) {
+        int i = ci + lane % 3 - 1, j = cj + (lane / 3) % 3 - 1, k = ck + lane / 9 - 1;
+        i += i < 0 ? pc.nc[0] : i >= pc.nc[0] ? -pc.nc[0] : 0;
+        j += j < 0 ? pc.nc[1] : j >= pc.nc[1] ? -pc.nc[1] : 0;
+        k += k < 0 ? pc.nc[2] : k >= pc.nc[2] ? -pc.nc[2] : 0;
+        const int c = i + (j + k * pc.nc[1]) * pc.nc[0];
+        beg = off[c];
+        cnt = off[c + 1] - beg;
+        sh.beg[lane] = beg;
+    }
+    int run = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
+    }
+    if (lane < 28) sh.pre[lane] = run - cnt;
+}
+
+// Candidates [first, first + count) of the block's list into shared memory,
+// padded to a multiple of 32 with positions that are never selected.
+__device__ __forceinline__ void fpp_stage(const PC& pc, const float4* __restrict__ spos, FppShared& sh, int first,
+                                          int count) {
+    const int padded = (count + 31) & ~31;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < padded; q += 32 * kFppWarps) {
+        float4 v = make_float4(INFINITY, 0.f, 0.f, __int_as_float(-1));
+        if (q < count) {
+            const int g = first + q;
+            int c = 0;  // the last cell whose prefix is <= g
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (c + step < 27 && sh.pre[c + step] <= g) c += step;
+            v = spos[sh.beg[c] + (g - sh.pre[c])];
+            v.x += (float)(c % 3 - 1) * pc.f_dc[0];
+            v.y += (float)((c / 3) % 3 - 1) * pc.f_dc[1];
+            v.z += (float)(c / 9 - 1) * pc.f_dc[2];
+        }
+        sh.cand[q] = v;
+    }
+}
+
+__device__ __forceinline__ bool any_force(const double* __restrict__ f, int n, int i) {
+    return nonzero_bits(f[i]) || nonzero_bits(f[n + i]) || nonzero_bits(f[2 * n + i]);
+}
+
+// Sums of four values over the warp: lanes 0, 8, 16, 24 get the totals of
+// v0, v1, v2, v3 (six additions a lane instead of twenty).
+template <typename TA> __device__ __forceinline__ TA warp_total4(TA v0, TA v1, TA v2, TA v3, int lane) {
+    const bool up = lane & 16, odd = lane & 8;
+    TA a = up ? v2 : v0, b = up ? v3 : v1;
+    a += __shfl_xor_sync(0xffffffffu, up ? v0 : v2, 16);
+    b += __shfl_xor_sync(0xffffffffu, up ? v1 : v3, 16);
+    TA t = odd ? b : a;
+    t += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// d = x_i - x_j by the minimum-image rule (cluster.cpp:225-232); |d| > thr on
+// the bits (non-negative doubles order like their bits).
+__device__ __forceinline__ double min_image(double d, double thr, double L) {
+    const long long m = __double_as_longlong(d) & 0x7fffffffffffffffll;
+    return m > __double_as_longlong(thr) ? d - copysign(L, d) : d;
+}
+
+// r_eq / |d| from s = |d|^2 / r_eq^2 > 0: an FP32 estimate y and one
+// third-order (Halley) step y (1 + e/2 + 3 e^2/8), e = 1 - s y^2, whose
+// remainder is below e^3: rounding only.  s outside the FP32 range (or NaN)
+// takes the library's square root and division.
+__device__ __forceinline__ double inv_distance(double s) {
+    const long long b = __double_as_longlong(s);
+    if (b < 0x3990000000000000ll || b >= 0x4660000000000000ll) return 1.0 / sqrt(s);  // 2^-102, 2^103
+    const double y = (double)rsqrtf((float)s);
+    const double e = fma(-(s * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Queues the staged candidates of home particle i (at h in the home frame)
+// and calls body(id) with full warps of them; `held` candidates stay queued.
+template <class Body>
+__device__ __forceinline__ void fpp_select(const PC& pc, const FppShared& sh, int* queue, float4 h, int count, int lane,
+                                           int& held, Body&& body) {
+    const int i = __float_as_int(h.w);
+    const unsigned below = (1u << lane) - 1u;
+    for (int q0 = 0; q0 < count; q0 += 32) {
+        const float4 c = sh.cand[q0 + lane];
+        const float dx = h.x - c.x, dy = h.y - c.y, dz = h.z - c.z;
+        const int j = __float_as_int(c.w);
+        // !(>): a NaN separation is passed on to the evaluation (padding, id -1, never is)
+        const bool take = !(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) > pc.f_req2_sel) && j != i && j >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (m == 0) continue;
+        if (take) queue[held + __popc(m & below)] = j;
+        held += __popc(m);
+        __syncwarp();
+        if (held >= 32) {
+            body(queue[lane]);
+            held -= 32;
+            const int rest = lane < held ? queue[32 + lane] : 0;
+            __syncwarp();
+            if (lane < held) queue[lane] = rest;
+            __syncwarp();
+        }
+    }
+}
+
+// The block's home particles, one per warp and round: body(i)'s pair functor
+// for every selected candidate, then done(i, ...).  blockIdx.x = cell,
+// blockIdx.y of gridDim.y shares of its particles.
+template <class Home>
+__device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict__ spos, const int* __restrict__ off,
+                                          Home&& home) {
+    __shared__ FppShared sh;
+    const int cell = blockIdx.x;
+    const int hb = off[cell], nh = off[cell + 1] - hb;
+    if ((int)blockIdx.y * kFppWarps >= nh) return;  // the whole block
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    fpp_cells(pc, cell, off, sh);
+    __syncthreads();
+    const int total = sh.pre[27];
+    bool staged = false;
+    for (int h0 = blockIdx.y * kFppWarps; h0 < nh; h0 += gridDim.y * kFppWarps) {
+        const bool on = h0 + w < nh;
+        const float4 h = spos[hb + (on ? h0 + w : 0)];
+        home(h, on, lane, [&](auto&& pair) {
+            int held = 0;
+            for (int first = 0; first < total; first += kFppStage) {
+                const int count = min(kFppStage, total - first);
+                if (!staged || total > kFppStage) {  // one round: staged once for all home particles
+                    __syncthreads();
+                    fpp_stage(pc, spos, sh, first, count);
+                    __syncthreads();
+                    staged = true;
+                }
+                if (on) fpp_select(pc, sh, sh.queue[w], h, count, lane, held, pair);
+            }
+            if (lane < held) pair(sh.queue[w][lane]);
+            __syncwarp();
+        });
+    }
+}
+
+template <typename TA>
+__global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const double* __restrict__ p,
+                                                              const float4* __restrict__ spos,
+                                                              const int4* __restrict__ ipos,
+                                                              const int* __restrict__ off,
+                                                              const double* __restrict__ rmp_p,
+                                                              const double* __restrict__ f_pi,
+                                                              const int* __restrict__ it_mark, double* f_pp,
+                                                              double* tau_part) {
+    const int n = pc.n;
+    bool mark = false;
+    if (f_pi != nullptr) {
+        const int m = *it_mark;
+        mark = m >= 0 && any_force(f_pi, n, m);
+    }
+    fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
+        const int i = __float_as_int(h.w);
+        const bool tau_on = mark && any_force(f_pi, n, i);
+        TA ax = TA(0), ay = TA(0), az = TA(0), tau = TA(0);
+        if constexpr (sizeof(TA) == sizeof(float)) {
+            const float req = pc.f_req, str = (float)*rmp_p * pc.f_kn;
+            const int4 hi = ipos[i];
+            walk([&](int j) {
+                const int4 c = ipos[j];
+                float dx = (float)(int)((unsigned)hi.x - (unsigned)c.x) * pc.f_unit[0];
+                float dy = (float)(int)((unsigned)hi.y - (unsigned)c.y) * pc.f_unit[1];
+                float dz = (float)(int)((unsigned)hi.z - (unsigned)c.z) * pc.f_unit[2];
+                float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                if (d2 == 0.f) {  // coincident
+                    double d[3];
+                    coincident_d(min(i, j), max(i, j), pc.r_p, d);
+                    const float sg = i < j ? 1.f : -1.f;
+                    dx = sg * (float)d[0];
+                    dy = sg * (float)d[1];
+                    dz = sg * (float)d[2];
+                    d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                }
+                // 1/|d|: the FP32 estimate and one Newton step
+                float y = rsqrtf(d2);
+                y = fmaf(0.5f * y, fmaf(-(d2 * y), y, 1.f), y);
+                const float dn = d2 * y;
+                if (!(dn < req)) return;
+                const float sc = (req - dn) * (str * y);  // the force is sc d
+                ax = fmaf(dx, sc, ax);
+                ay = fmaf(dy, sc, ay);
+                az = fmaf(dz, sc, az);
+                if (tau_on && i < j) tau = fmaf(0.5f * sc, d2, tau);
+            });
+        } else {
+            const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
+            const double str = *rmp_p * pc.k_n;
+            walk([&](int j) {
+                double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
+                               min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
+                double d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+                if (!nonzero_bits(d2) && !nonzero_bits(d[0]) && !nonzero_bits(d[1]) && !nonzero_bits(d[2])) {
+                    coincident_d(min(i, j), max(i, j), pc.r_p, d);
+                    if (j < i)
+                        for (int a = 0; a < 3; ++a) d[a] = -d[a];
+                    d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+                }
+                // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
+                const double sc = fma(inv_distance(d2 * pc.inv_req2), str, -str);
+                if (!(sc > 0.0)) return;
+                ax = fma(d[0], sc, ax);
+                ay = fma(d[1], sc, ay);
+                az = fma(d[2], sc, az);
+                if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
+            });
+        }
+        const TA t = warp_total4(ax, ay, az, tau, lane);
+        if (on && (lane & 7) == 0) {
+            if (lane < 24) f_pp[(lane >> 3) * n + i] = (double)t;
+            else if (tau_part) tau_part[i] = (double)t;
+        }
+    });
+}
+
+// Blocks per home cell: enough that every SM has several.
+static dim3 fpp_grid(const fipi_ctx* ctx) {
+    const ParticleBufs& b = ctx->pb;
+    const int per_cell = b.n / b.ncells + 1;
+    int shares = (4 * ctx->num_sms + b.ncells - 1) / b.ncells;
+    shares = std::min(shares, (per_cell + kFppWarps - 1) / kFppWarps);
+    return dim3(b.ncells, std::max(1, shares));
 }
 
 // it_mark of cluster::sorting (cluster.cpp:128-138): the first index of
@@ -1339,9 +1624,6 @@ void particles_spread(fipi_ctx* ctx) {
     }
 }
 
-// compute_f_pp; with `tau` the packing energy of cluster.cpp:256-259 is
-// accumulated per particle and summed in a fixed order.  TA = float with
-// at least 4 cells per axis takes the FP32 cell-relative path.
 // it_mark for the packing energy: the first index of the largest p_y.
 static void it_mark_launch(fipi_ctx* ctx, const double* p) {
     ParticleBufs& b = ctx->pb;
@@ -1353,10 +1635,24 @@ static void it_mark_launch(fipi_ctx* ctx, const double* p) {
 
 // compute_f_pp; with `tau` the packing energy of cluster.cpp:256-259 is
 // accumulated per particle (tau_part) and summed when it is asked for.
-// TA = float with at least 4 cells per axis takes the FP32 cell-relative path.
-static bool f_pp_fast_path(const fipi_ctx* ctx, bool fp32) {
+//
+// Mixed form with at least 4 cells per axis: k_f_pp_fast.  The FP64 form, and
+// 3 cells on an axis: k_f_pp_warp wherever its cell offsets give the minimum
+// image (see there); otherwise (margin != 0, 3 cells on an axis and r_eq >
+// d_cell, r_eq >= L/2) k_f_pp, one warp per home cell in the reference's pair
+// order.  Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp
+// 110; 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 12; mixed,
+// 20,000 particles, k_f_pp_fast 27, k_f_pp_warp 32.
+enum class FppPath { cell, warp, fast };
+static FppPath f_pp_path(const fipi_ctx* ctx, bool fp32) {
     const ParticleBufs& b = ctx->pb;
-    return fp32 && b.ncell[0] >= 4 && b.ncell[1] >= 4 && b.ncell[2] >= 4;
+    if (fp32 && b.ncell[0] >= 4 && b.ncell[1] >= 4 && b.ncell[2] >= 4) return FppPath::fast;
+    const double L[3] = {ctx->P.lx, ctx->P.ly, ctx->P.lz};
+    if (ctx->P.margin != 0.0) return FppPath::cell;
+    for (int a = 0; a < 3; ++a)
+        if (b.ncell[a] < 3 || (b.ncell[a] == 3 && ctx->P.r_eq > b.dcell[a]) || !(ctx->P.r_eq < 0.5 * L[a]))
+            return FppPath::cell;
+    return FppPath::warp;
 }
 
 template <typename TA>
@@ -1364,16 +1660,22 @@ static void f_pp_launch(fipi_ctx* ctx, const double* p, const double* rmp, const
                         bool have_it_mark = false, bool have_spos = false) {
     ParticleBufs& b = ctx->pb;
     const PC pc = make_pc(ctx);
-    const int warps = b.ncells;
-    const int blocks = (warps * 32 + 255) / 256;
     if (tau && !have_it_mark) it_mark_launch(ctx, p);
-    const bool fast = f_pp_fast_path(ctx, sizeof(TA) == sizeof(float));
-    if (fast) {
-        if (!have_spos) { LaunchScope ls_(ctx, "sorted FP32 positions", 0.0); k_sorted_pos<<<(b.n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, b.keys, b.ids, b.spos); }
-        { LaunchScope ls_(ctx, "contact forces (warp per cell)", 0.0); k_f_pp_fast<<<b.ncells, 32 * kFppRows, 0, ctx->stream>>>(pc, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp, b.tau_part); }
+    const FppPath path = f_pp_path(ctx, sizeof(TA) == sizeof(float));
+    if (path != FppPath::cell) {
+        if (!have_spos) { LaunchScope ls_(ctx, "sorted FP32 positions", 0.0); k_sorted_pos<<<(b.n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, b.keys, b.ids, b.spos, b.ipos); }
+        LaunchScope ls_(ctx, "contact forces", 0.0);
+        if (path == FppPath::fast)
+            k_f_pp_fast<<<b.ncells, 32 * kFppRows, 0, ctx->stream>>>(pc, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr,
+                                                                     b.it_mark, f_pp, tau ? b.tau_part : nullptr);
+        else
+            k_f_pp_warp<TA><<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
+                pc, p, b.spos, b.ipos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp,
+                tau ? b.tau_part : nullptr);
     } else {
+        const int blocks = (b.ncells * 32 + 255) / 256;
         { LaunchScope ls_(ctx, "contact forces (warp per cell)", 0.0); k_f_pp<TA, 0><<<blocks, 256, 0, ctx->stream>>>(pc, p, b.ids, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark,
-                                                  f_pp, b.tau_part, nullptr, nullptr, nullptr); }
+                                                  f_pp, tau ? b.tau_part : nullptr, nullptr, nullptr, nullptr); }
     }
     b.tau_valid = tau;
 }
@@ -1429,7 +1731,7 @@ template <typename T> static void step_t(fipi_ctx* ctx) {
     const T* g0 = (const T*)ctx->fb.g[0];
     const T* g1 = (const T*)ctx->fb.g[1];
     const T* g2 = (const T*)ctx->fb.g[2];
-    float4* spos = f_pp_fast_path(ctx, FAST) ? b.spos : nullptr;
+    float4* spos = f_pp_path(ctx, FAST) != FppPath::cell ? b.spos : nullptr;
     // per stage: interpolate_local_variables, sorting, compute_f_pi,
     // compute_f_pp(t+1), compute_f_ext (zero), advect, enforce_bc
     // (main.cpp:198-217); the ramp(t+1, 0.2 t_end) factor is kept on the
@@ -1516,6 +1818,8 @@ fipi_status particles_alloc(fipi_ctx* ctx) {
     FIPI_CUDA(ctx, A((void**)&b.hist, sizeof(unsigned) * b.hist_cap));
     FIPI_CUDA(ctx, A((void**)&b.tau_part, sizeof(double) * n));
     FIPI_CUDA(ctx, A((void**)&b.spos, sizeof(float4) * n));
+    // the mixed form's k_f_pp_warp reads box fractions instead of the FP64 positions
+    if (ctx->prec == FIPI_MIXED && f_pp_path(ctx, true) == FppPath::warp) FIPI_CUDA(ctx, A((void**)&b.ipos, sizeof(int4) * n));
     FIPI_CUDA(ctx, A((void**)&b.sp_fw, sizeof(double) * 6 * n));
     FIPI_CUDA(ctx, A((void**)&b.ymax, sizeof(unsigned long long) * 2));
     {
@@ -1533,7 +1837,7 @@ void particles_free(fipi_ctx* ctx) {
     ParticleBufs& b = ctx->pb;
     void* all[] = {b.p, b.p_old, b.u_old, b.f_pp, b.f_pi, b.r, b.cth, b.keys, b.keys_alt, b.ids, b.ids_alt,
                    b.cell_off, b.cell_cnt, b.sp_keys, b.sp_keys_alt, b.sp_vals, b.sp_vals_alt, b.sp_prev,
-                   b.hist, b.tau_part, b.it_mark, b.tau, b.spos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
+                   b.hist, b.tau_part, b.it_mark, b.tau, b.spos, b.ipos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
     for (void* p : all)
         if (p) cudaFree(p);
     b = ParticleBufs{};
@@ -2042,10 +2346,57 @@ __global__ void k_adj_stage(PC pc, int stage, const double* __restrict__ p, cons
 // and |d| < r_eq test), lam_p[i] += J(d) (lamF[i] - lamF[j]) with
 // J = ramp k_n ((r_eq/|d| - 1) I - r_eq d d^T / |d|^3), which is even in d.
 // With respect to k_n: pkn[i] += lamF[i] . (force on i) / k_n, the force on
-// i being +F(d) when i < j and -F(d) otherwise (f_pp[it] += F, f_pp[id] -= F,
-// cluster.cpp:246-255), F(d) = (r_eq - |d|) ramp k_n d / |d|.
-// Warp per home cell, lane per home particle as in k_f_pp; coincident pairs
-// (random separation in the reference) contribute nothing.
+// i being F(d) with d = p_i - p_j for either id order (f_pp[it] += F,
+// f_pp[id] -= F, cluster.cpp:246-255), F(d) = (r_eq - |d|) ramp k_n d / |d|.
+// Coincident pairs (random separation in the reference) contribute nothing.
+// The terms of one pair, added to acc (lam_p[i]) and acc_kn (pkn[i]); d is
+// p_i - p_j by the minimum-image rule, li = lamF[i].  The k_n term
+// lamF[i] . (force on i) / k_n is F(d) . li / k_n.
+__device__ __forceinline__ void pair_adj(const PC& pc, const double d[3], const double li[3],
+                                         const double* __restrict__ lamF, int j, double rmp, double acc[3],
+                                         double& acc_kn) {
+    const int n = pc.n;
+    const double s = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0])) * pc.inv_req2;
+    if (!nonzero_bits(s)) return;
+    const double q = inv_distance(s);  // r_eq / |d|
+    const double g = q - 1.0;
+    if (!(g > 0.0)) return;
+    const double dl[3] = {li[0] - lamF[j], li[1] - lamF[n + j], li[2] - lamF[2 * n + j]};
+    const double sc = rmp * pc.k_n, a = sc * g;
+    const double b = (sc * q) * (q * q * pc.inv_req2) * fma(d[2], dl[2], fma(d[1], dl[1], d[0] * dl[0]));
+    for (int e = 0; e < 3; ++e) acc[e] = fma(a, dl[e], fma(-b, d[e], acc[e]));
+    acc_kn = fma(g * rmp, fma(d[2], li[2], fma(d[1], li[1], d[0] * li[0])), acc_kn);
+}
+
+// One warp per home particle, FP32 selection (k_f_pp_warp).
+__global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_adj_warp(PC pc, const double* __restrict__ p,
+                                                                  const float4* __restrict__ spos,
+                                                                  const int* __restrict__ off,
+                                                                  const double* __restrict__ rmp_p,
+                                                                  const double* __restrict__ lamF, double* lam_p,
+                                                                  double* pkn) {
+    const int n = pc.n;
+    const double rmp = *rmp_p;
+    fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
+        const int i = __float_as_int(h.w);
+        const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
+        const double li[3] = {lamF[i], lamF[n + i], lamF[2 * n + i]};
+        double acc[3] = {0.0, 0.0, 0.0}, acc_kn = 0.0;
+        walk([&](int j) {
+            const double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
+                                 min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
+            pair_adj(pc, d, li, lamF, j, rmp, acc, acc_kn);
+        });
+        const double t = warp_total4(acc[0], acc[1], acc[2], acc_kn, lane);
+        if (on && (lane & 7) == 0) {
+            if (lane < 24) lam_p[(lane >> 3) * n + i] += t;
+            else pkn[i] += t;
+        }
+    });
+}
+
+// One warp per home cell, lane per home particle (k_f_pp), for the cases
+// k_f_pp_warp does not take.
 __global__ void k_f_pp_adj(PC pc, const double* __restrict__ p, const unsigned* __restrict__ ids,
                            const int* __restrict__ off, const double* __restrict__ rmp_p,
                            const double* __restrict__ lamF, double* lam_p, double* pkn) {
@@ -2056,16 +2407,12 @@ __global__ void k_f_pp_adj(PC pc, const double* __restrict__ p, const unsigned* 
     const int n = pc.n;
     const int ci = cell % pc.nc[0], cj = (cell / pc.nc[0]) % pc.nc[1], ck = cell / (pc.nc[0] * pc.nc[1]);
     const int beg = off[cell], end = off[cell + 1];
-    const double T0 = pc.dc[0] * (pc.nc[0] - 2), T1 = pc.dc[1] * (pc.nc[1] - 2), T2 = pc.dc[2] * (pc.nc[2] - 2);
-    const double sc = (*rmp_p) * pc.k_n;
-    for (int base = beg; base < end; base += 32) {
-        const int s = base + lane;
-        const bool active = s < end;
-        const int i = active ? (int)ids[s] : 0;
+    const double rmp = *rmp_p;
+    for (int s = beg + lane; s < end; s += 32) {
+        const int i = (int)ids[s];
         const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
         const double li[3] = {lamF[i], lamF[n + i], lamF[2 * n + i]};
-        double acc[3] = {0.0, 0.0, 0.0};
-        double acc_kn = 0.0;
+        double acc[3] = {0.0, 0.0, 0.0}, acc_kn = 0.0;
         for (int dk = -1; dk <= 1; ++dk)
             for (int dj = -1; dj <= 1; ++dj)
                 for (int di = -1; di <= 1; ++di) {
@@ -2074,37 +2421,15 @@ __global__ void k_f_pp_adj(PC pc, const double* __restrict__ p, const unsigned* 
                     const int qe = off[co + 1];
                     for (int q = off[co]; q < qe; ++q) {
                         const int j = (int)ids[q];
-                        if (!active || j == i) continue;
-                        double d[3];
-                        if (i < j) {
-                            d[0] = xi - p[j];
-                            d[1] = yi - p[n + j];
-                            d[2] = zi - p[2 * n + j];
-                        } else {
-                            d[0] = p[j] - xi;
-                            d[1] = p[n + j] - yi;
-                            d[2] = p[2 * n + j] - zi;
-                        }
-                        if (d[0] > T0) d[0] = d[0] - pc.L[0];
-                        else if (d[0] < -T0) d[0] = d[0] + pc.L[0];
-                        if (d[1] > T1) d[1] = d[1] - pc.L[1];
-                        else if (d[1] < -T1) d[1] = d[1] + pc.L[1];
-                        if (d[2] > T2) d[2] = d[2] - pc.L[2];
-                        else if (d[2] < -T2) d[2] = d[2] + pc.L[2];
-                        const double dn = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-                        if (!(dn < pc.r_eq) || dn == 0.0) continue;
-                        const double dl[3] = {li[0] - lamF[j], li[1] - lamF[n + j], li[2] - lamF[2 * n + j]};
-                        const double a = pc.r_eq / dn - 1.0;
-                        const double b = pc.r_eq / (dn * dn * dn) * (d[0] * dl[0] + d[1] * dl[1] + d[2] * dl[2]);
-                        for (int e = 0; e < 3; ++e) acc[e] += sc * (a * dl[e] - b * d[e]);
-                        const double fk = (pc.r_eq - dn) * (*rmp_p) / dn * (d[0] * li[0] + d[1] * li[1] + d[2] * li[2]);
-                        acc_kn += (i < j) ? fk : -fk;
+                        if (j == i) continue;
+                        const double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]),
+                                             min_image(yi - p[n + j], pc.img[1], pc.L[1]),
+                                             min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
+                        pair_adj(pc, d, li, lamF, j, rmp, acc, acc_kn);
                     }
                 }
-        if (active) {
-            for (int e = 0; e < 3; ++e) lam_p[e * n + i] += acc[e];
-            pkn[i] += acc_kn;
-        }
+        for (int e = 0; e < 3; ++e) lam_p[e * n + i] += acc[e];
+        pkn[i] += acc_kn;
     }
 }
 
@@ -2224,11 +2549,21 @@ fipi_status particles_adjoint(fipi_ctx* ctx) {
     const double* g0 = (const double*)ctx->fb.g[0];
     const double* g1 = (const double*)ctx->fb.g[1];
     const double* g2 = (const double*)ctx->fb.g[2];
-    const int cells_blocks = (b.ncells * 32 + 255) / 256;
     // stage 1 recomputed at p^n: interpolation, f_pi, contact forces, p1
     { LaunchScope ls_(ctx, "adjoint: interpolate + f_pi", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.tp0, c, g0, g1, g2, b.r, b.cth, a.loc, a.fpi1); }
-    build_cells(ctx, a.tp0);
-    { LaunchScope ls_(ctx, "adjoint: contact forces", 0.0); k_f_pp<double, 0><<<cells_blocks, 256, 0, ctx->stream>>>(pc, a.tp0, b.ids, b.cell_off, a.rmp, nullptr, b.it_mark, a.fpp1, nullptr, nullptr, nullptr, nullptr); }
+    // the contact forces and their adjoint at positions q
+    float4* spos = f_pp_path(ctx, false) != FppPath::cell ? b.spos : nullptr;
+    auto contact_adj = [&](const double* q, const double* lamF, double* lam_p) {
+        LaunchScope ls_(ctx, "adjoint: contact forces", 0.0);
+        if (spos)
+            k_f_pp_adj_warp<<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(pc, q, spos, b.cell_off, a.rmp, lamF,
+                                                                               lam_p, a.pp_kn);
+        else
+            k_f_pp_adj<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, q, b.ids, b.cell_off, a.rmp, lamF,
+                                                                             lam_p, a.pp_kn);
+    };
+    build_cells(ctx, a.tp0, false, spos);
+    f_pp_launch<double>(ctx, a.tp0, a.rmp, nullptr, a.fpp1, false, false, spos != nullptr);
     { LaunchScope ls_(ctx, "adjoint: advect", 0.0); k_adj_advect1<<<nb, 256, 0, ctx->stream>>>(pc, a.tp0, a.fpi1, a.fpp1, b.r, a.p1); }
     { LaunchScope ls_(ctx, "adjoint: interpolate", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.p1, c, g0, g1, g2, b.r, b.cth, a.loc + 4 * n, nullptr); }
     // stage 2 reversed at p1
@@ -2236,12 +2571,12 @@ fipi_status particles_adjoint(fipi_ctx* ctx) {
     FIPI_CUDA(ctx, cudaMemsetAsync(a.pp_sig, 0, sizeof(double) * n, ctx->stream));
     FIPI_CUDA(ctx, cudaMemsetAsync(a.pp_kn, 0, sizeof(double) * n, ctx->stream));
     { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 2, a.p1, c, g0, g1, g2, a.loc + 4 * n, b.r, b.cth, a.la_p, a.la_fpp, nullptr, a.lamF2, a.lamloc + 4 * n, a.lam_p1, a.dct, a.pp_sig); }
-    build_cells(ctx, a.p1);
-    { LaunchScope ls_(ctx, "adjoint: contact forces", 0.0); k_f_pp_adj<<<cells_blocks, 256, 0, ctx->stream>>>(pc, a.p1, b.ids, b.cell_off, a.rmp, a.lamF2, a.lam_p1, a.pp_kn); }
+    build_cells(ctx, a.p1, false, spos);
+    contact_adj(a.p1, a.lamF2, a.lam_p1);
     // stage 1 reversed at p^n (la_p becomes the start-state cotangent)
     { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 1, a.tp0, c, g0, g1, g2, a.loc, b.r, b.cth, a.la_p, nullptr, a.lam_p1, a.lamF1, a.lamloc, a.la_p, a.dct, a.pp_sig); }
-    build_cells(ctx, a.tp0);
-    { LaunchScope ls_(ctx, "adjoint: contact forces", 0.0); k_f_pp_adj<<<cells_blocks, 256, 0, ctx->stream>>>(pc, a.tp0, b.ids, b.cell_off, a.rmp, a.lamF1, a.la_p, a.pp_kn); }
+    build_cells(ctx, a.tp0, false, spos);
+    contact_adj(a.tp0, a.lamF1, a.la_p);
     param_acc(ctx, a.pp_sig, n, 1.0, a.pg + kPgSigmaAttach);
     param_acc(ctx, a.pp_kn, n, 1.0, a.pg + kPgKn);
     // interpolation adjoint onto the grid: part = [c, g0, g1, g2] cotangents
