@@ -14,10 +14,9 @@
 // The inverse runs Z, Y, X(C2R).  Element-wise work is fused into the X
 // passes (real space) and the Z passes (spectral space) through functors.
 //
-// The row FFT is an in-place radix-4 Stockham autosort in shared memory
-// (one radix-2 stage first when log2 n is odd), four elements per thread
-// per stage, twiddles from a table exp(-2 pi i q / n) computed on the host
-// in extended precision.  An R2C row of length nx is a complex FFT of
+// The row FFTs are register codelets with exchanges through shared memory
+// (fft2.cuh), twiddles from a table exp(-2 pi i q / n) computed on the host in
+// extended precision; the FP64 form transforms in block fixed point (fx64.cuh).  An R2C row of length nx is a complex FFT of
 // length M over (x[2n], x[2n+1]) pairs plus the standard split
 // post-processing; C2R is the mirror image.  Unnormalised, like FFTW.
 #pragma once
@@ -45,6 +44,10 @@ template <typename T> struct Tiles {
     static constexpr int TY = 128 / (2 * sizeof(T));  // 16 (fp32) / 8 (fp64)
     static constexpr int TZ = 128 / (2 * sizeof(T));
 };
+
+// Twiddle table of the passes: the FP64 form's transforms run in block fixed
+// point.
+template <typename T> using tw_t = typename std::conditional<sizeof(T) == sizeof(double), longlong2, cplx<T>>::type;
 
 // A Z-pass operation that declares PreT and pre() has global reads in its
 // mid operation that can be issued ahead (k_zpass_rt batches ZU modes; two
@@ -106,7 +109,7 @@ template <typename T> struct YGroups {
 // first_wait: polls of the block's first copy wait (-1: the normal bound);
 // a test hook that lets the bounded-wait error path run (fipi_set_debug).
 template <typename T, int DIR, int N>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_ypass_tma(Geom g, const cplx<T>* __restrict__ twy, FieldPtrs<T> fp,
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_ypass_tma(Geom g, const tw_t<T>* __restrict__ twy, FieldPtrs<T> fp,
                                                        int fields, int* status, int first_wait) {
     using C = cplx<T>;
     constexpr int EM = YE<T>::value;
@@ -122,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_ypass_tma(
     C* buf0 = reinterpret_cast<C*>(smem_raw);
     __shared__ __align__(8) uint64_t bar[S];
     __shared__ int abort_flag;
+    __shared__ FxSlot wsize[kThreads / 32];  // FP64: sizes of the warps' rows (rows of more than 32 threads)
     const int tid = threadIdx.x;
     const long long rows_f = (long long)g.nz * g.h;
     const long long tiles_f = (rows_f + RB - 1) / RB;
@@ -189,8 +193,28 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_ypass_tma(
 #pragma unroll
                 for (int i = 0; i < IO::E; ++i) v[i] = in[row * N + IO::in_elem(t, i)];
             }
-            __syncthreads();  // the round's exchange rows overlap its natural rows
-            smem_fft2<T, DIR, N, true, true, EM>(in + gr * RG * PITCH, xidx, rl, t, act, twy, 1, v);
+            if constexpr (sizeof(T) == sizeof(double)) {
+                FxSize z;
+                if (act)
+#pragma unroll
+                    for (int i = 0; i < IO::E; ++i) z.add(v[i]);
+                z = fx_row_size<Tn>(z);
+                if constexpr (Tn > 32)
+                    if ((tid & 31) == 0) wsize[tid >> 5] = FxSlot{z.mag, z.l1};
+                __syncthreads();  // the round's exchange rows overlap its natural rows
+                if constexpr (Tn > 32) {
+                    z = FxSize{};
+#pragma unroll
+                    for (int k = 0; k < Tn / 32; ++k) {
+                        z.mag = max(z.mag, wsize[rl * (Tn / 32) + k].mag);
+                        z.l1 += wsize[rl * (Tn / 32) + k].l1;
+                    }
+                }
+                fx_fft_regs<DIR, N, false>(in + gr * RG * PITCH, xidx, rl, t, act, twy, 1, z, v);
+            } else {
+                __syncthreads();  // the round's exchange rows overlap its natural rows
+                smem_fft2<T, DIR, N, true, true, EM>(in + gr * RG * PITCH, xidx, rl, t, act, twy, 1, v);
+            }
             if (act) {
                 C* out = fp.pick(fp.out, f) + (r0 + row) * N;
 #pragma unroll
@@ -228,8 +252,9 @@ template <typename T> __host__ __device__ inline int zpass_threads(int nz) {
 }
 
 template <typename T, int NF, int DIR, int N, class Op>
-__global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const cplx<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
+    constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     constexpr int EM = FftE<T>::value;
     constexpr int E = N < EM ? N : EM;
     constexpr int Tn = N / E;
@@ -243,6 +268,16 @@ __global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const cplx<T>* __res
     const size_t base = (size_t)kx * g.ny + ky;
     const IdxColumns idx{TZ};
     constexpr size_t fstride = (size_t)N * TZ;
+    constexpr int NT = TZ * Tn;
+    __shared__ FxSlot slot[FX ? 2 : 1][FX ? (NT + 31) / 32 * TZ : 1];
+    // FP64: field f from the tile and back into it
+    auto fx_field = [&](auto f) {
+        C v[E];
+        fx_fft_column<DIR, N, TZ, NT>(s + f * fstride, idx, c, t, twz, slot[f & 1], v);
+        using IO = FftIO<T, DIR, N>;
+#pragma unroll
+        for (int i = 0; i < E; ++i) s[f * fstride + idx(c, IO::out_elem(t, i))] = v[i];
+    };
     if constexpr (NF == 1) {
         // the loaded modes are exactly the first stage's inputs
         using IO = FftIO<T, DIR, N>;
@@ -254,7 +289,21 @@ __global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const cplx<T>* __res
             op.load(kx, ky, z, base + z * zstride, w);
             v[i] = w[0];
         }
-        smem_fft2<T, DIR, N, true, false>(s, idx, c, t, true, twz, 1, v);
+        if constexpr (FX) {
+            FxSize z;
+#pragma unroll
+            for (int i = 0; i < E; ++i) z.add(v[i]);
+            z = fx_column_size<TZ, NT>(z, slot[0]);
+            fx_fft_regs<DIR, N, false>(s, idx, c, t, true, twz, 1, z, v);
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                const int z = IO::out_elem(t, i);
+                op.store(kx, ky, z, base + z * zstride, &v[i]);
+            }
+            return;
+        } else {
+            smem_fft2<T, DIR, N, true, false>(s, idx, c, t, true, twz, 1, v);
+        }
     } else if constexpr (HasSrc<Op>::value) {
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
@@ -268,7 +317,10 @@ __global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const cplx<T>* __res
         cp_async_wait_all();
         __syncthreads();
 #pragma unroll
-        for (int f = 0; f < NF; ++f) smem_fft2<T, DIR, N>(s + f * fstride, idx, c, t, true, twz, 1);
+        for (int f = 0; f < NF; ++f) {
+            if constexpr (FX) fx_field(f);
+            else smem_fft2<T, DIR, N>(s + f * fstride, idx, c, t, true, twz, 1);
+        }
     } else {
         // loads in chunks of CH modes per thread: CH * NF independent loads in flight
         constexpr int CH = 8 / NF >= 2 ? 8 / NF : 2;
@@ -291,7 +343,10 @@ __global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const cplx<T>* __res
         }
         __syncthreads();
 #pragma unroll
-        for (int f = 0; f < NF; ++f) smem_fft2<T, DIR, N>(s + f * fstride, idx, c, t, true, twz, 1);
+        for (int f = 0; f < NF; ++f) {
+            if constexpr (FX) fx_field(f);
+            else smem_fft2<T, DIR, N>(s + f * fstride, idx, c, t, true, twz, 1);
+        }
     }
 #pragma unroll 4
     for (int i = 0; i < E; ++i) {
@@ -337,8 +392,9 @@ template <bool PAD> struct IdxZ {
 // the mid operation walk the tile with ky fastest (full runs per warp).
 // Tiles whose load() only copies arrays (src()) arrive by cp.async.
 template <typename T, int NF, int NB, int DIR, int N, int COLS, class Op, int EM = FftE<T>::value>
-__global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const cplx<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
+    constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     using SH = ZRtShape<T, N, COLS, EM>;
     constexpr int RC = SH::RC, P = SH::P, NT = SH::THREADS;
     constexpr int ELEMS = COLS * N;
@@ -375,6 +431,8 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const cplx<T>* __
         __syncthreads();
     }
     const int cl = tid % RC, t = tid / RC;
+    __shared__ FxSlot slot[FX ? 2 : 1][FX ? (NT + 31) / 32 * RC : 1];
+    int turn = 0;
     // WZ: the forward transforms (and the first stage of each inverse) run
     // on columns owned by single warps (wc = tid / Tn), synchronising only
     // the warp; the mid operation and the inverse's last stage keep the
@@ -389,7 +447,17 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const cplx<T>* __
         }
         if constexpr (WZ) smem_fft2<T, DIR, N, EM, true>(s + f * fstride, idx, wc, wt, true, twz, 1);
         else
-            for (int r = 0; r < COLS; r += RC) smem_fft2<T, DIR, N, EM>(s + f * fstride + r, idx, cl, t, true, twz, 1);
+            for (int r = 0; r < COLS; r += RC) {
+                if constexpr (FX) {
+                    C v[SH::E];
+                    fx_fft_column<DIR, N, RC, NT>(s + f * fstride + r, idx, cl, t, twz, slot[turn ^= 1], v);
+                    using IOF = FftIO<T, DIR, N, EM>;
+#pragma unroll
+                    for (int i = 0; i < SH::E; ++i) s[f * fstride + r + idx(cl, IOF::out_elem(t, i))] = v[i];
+                } else {
+                    smem_fft2<T, DIR, N, EM>(s + f * fstride + r, idx, cl, t, true, twz, 1);
+                }
+            }
     }
     __syncthreads();
     if constexpr (HasPre<Op>::value) {
@@ -440,6 +508,8 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const cplx<T>* __
                 fft_stage<T, R0, -DIR, N, 1, false, false, EM, true>(s + b * fstride, idx, wc, wt, true, twz, 1, v);
                 __syncthreads();
                 fft_stages<T, -DIR, N, 1, R0, false, true, EM, false>(s + b * fstride, idx, cl, t, true, twz, 1, v);
+            } else if constexpr (FX) {
+                fx_fft_column<-DIR, N, RC, NT>(s + b * fstride + r, idx, cl, t, twz, slot[turn ^= 1], v);
             } else {
                 smem_fft2<T, -DIR, N, false, true, EM>(s + b * fstride + r, idx, cl, t, true, twz, 1, v);
             }
@@ -460,8 +530,9 @@ template <typename T, int N, int COLS, int EM = FftE<T>::value> struct ZRtShapeT
 };
 
 template <typename T, int NF, int NB, int DIR, int N, int COLS, class Op, int EM = FftE<T>::value>
-__global__ void __launch_bounds__(kThreads) k_zpass_rt_t(Geom g, const cplx<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(kThreads) k_zpass_rt_t(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
+    constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     using SH = ZRtShapeT<T, N, COLS, EM>;
     constexpr int E = SH::E, Tn = SH::Tn, TZ = SH::TZ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -495,8 +566,21 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt_t(Geom g, const cplx<T>* 
         }
     }
     __syncthreads();
+    constexpr int NT = TZ * Tn;
+    __shared__ FxSlot slot[FX ? 2 : 1][FX ? (NT + 31) / 32 * TZ : 1];
+    int turn = 0;
 #pragma unroll
-    for (int f = 0; f < NF; ++f) smem_fft2<T, DIR, N, EM>(s + f * fstride, idx, c, t, true, twz, 1);
+    for (int f = 0; f < NF; ++f) {
+        if constexpr (FX) {
+            C v[E];
+            fx_fft_column<DIR, N, TZ, NT>(s + f * fstride, idx, c, t, twz, slot[turn ^= 1], v);
+            using IOF = FftIO<T, DIR, N, EM>;
+#pragma unroll
+            for (int i = 0; i < E; ++i) s[f * fstride + idx(c, IOF::out_elem(t, i))] = v[i];
+        } else {
+            smem_fft2<T, DIR, N, EM>(s + f * fstride, idx, c, t, true, twz, 1);
+        }
+    }
     // each thread's outputs of the last stage are the modes z = t + Tn i
 #pragma unroll 2
     for (int i = 0; i < E; ++i) {
@@ -510,7 +594,21 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt_t(Geom g, const cplx<T>* 
     }
     __syncthreads();
 #pragma unroll
-    for (int b = 0; b < NB; ++b) smem_fft2<T, -DIR, N, EM>(s + b * fstride, idx, c, t, true, twz, 1);
+    for (int b = 0; b < NB; ++b) {
+        if constexpr (FX) {
+            C v[E];
+            fx_fft_column<-DIR, N, TZ, NT>(s + b * fstride, idx, c, t, twz, slot[turn ^= 1], v);
+            using IOI = FftIO<T, -DIR, N, EM>;
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                const int z = IOI::out_elem(t, i);
+                op.rr_store(b, base + z * zstride, v[i]);
+            }
+        } else {
+            smem_fft2<T, -DIR, N, EM>(s + b * fstride, idx, c, t, true, twz, 1);
+        }
+    }
+    if constexpr (!FX)
 #pragma unroll 4
     for (int i = 0; i < E; ++i) {
         const int z = t + Tn * i;
@@ -530,7 +628,7 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt_t(Geom g, const cplx<T>* 
 // keeps between the transforms), rr_mid (NF transformed values -> State),
 // rr_out (output b of a State) and rr_store (output b at gi).
 template <typename T, int NF, int NB, int DIR, int N, int COLS, class Op, int EM = FftE<T>::value>
-__global__ void __launch_bounds__(kThreads, 2) k_zpass_rr(Geom g, const cplx<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(kThreads, 2) k_zpass_rr(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
     using SH = ZRtShapeT<T, N, COLS, EM>;
     using IOF = FftIO<T, DIR, N, EM>;

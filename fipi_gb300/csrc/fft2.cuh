@@ -16,12 +16,14 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fx64.cuh"
 
 namespace fipi {
 
-// a * w, or a * conj(w) for the inverse direction
+// a * w, or a * conj(w) for the inverse direction (block fixed point: / 4)
 template <int DIR, typename C> __device__ __forceinline__ C mulw(C a, C w) {
-    return DIR < 0 ? mkc<C>(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x)
+    if constexpr (is_fx<C>) return fx_mulw<DIR>(a, w);
+    else return DIR < 0 ? mkc<C>(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x)
                    : mkc<C>(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
 }
 
@@ -43,6 +45,7 @@ template <int DIR, int E16, typename C> __device__ __forceinline__ C tw16(C a) {
     else if constexpr (e == 4) return cmul_i(a, DIR);
     else if constexpr (e == 8) return mkc<C>(-a.x, -a.y);
     else if constexpr (e == 12) return cmul_i(a, -DIR);
+    else if constexpr (is_fx<C>) return fx_rot8<DIR, e>(a);
     else {
         // exp(DIR 2 pi i e/16): forward (DIR < 0) uses (cos, -sin)
         constexpr double cs = cos16(e), sn = cos16((e + 12) & 15);  // sin(x) = cos(x - pi/2)
@@ -195,6 +198,7 @@ __device__ __forceinline__ void fft_stage(cplx<T>* s, const Idx& idx, int row, i
             const int k = g & (P - 1);
             if constexpr (P > 1) {
                 const int base = (NR / P) * k * ts;
+                if constexpr (is_fx<cplx<T>>) v[q * R] = fx_quarter(v[q * R]);  // the factor of mulw
 #pragma unroll
                 for (int m = 1; m < R; ++m) v[q * R + m] = mulw<DIR>(v[q * R + m], tw[m * base]);
             }
@@ -256,18 +260,47 @@ __device__ __forceinline__ void smem_fft2(cplx<T>* s, const Idx& idx, int row, i
     fft_stages<T, DIR, N, 0, 1, false, false, EM, WS>(s, idx, row, t, act, tw, ts, v);
 }
 
-// Calls f(std::integral_constant<int, n>) for a power of two n in [8, 512].
-template <class F> inline void dispatch_pow2(int n, F&& f) {
-    switch (n) {
-        case 4: f(std::integral_constant<int, 4>{}); break;
-        case 8: f(std::integral_constant<int, 8>{}); break;
-        case 16: f(std::integral_constant<int, 16>{}); break;
-        case 32: f(std::integral_constant<int, 32>{}); break;
-        case 64: f(std::integral_constant<int, 64>{}); break;
-        case 128: f(std::integral_constant<int, 128>{}); break;
-        case 256: f(std::integral_constant<int, 256>{}); break;
-        default: f(std::integral_constant<int, 512>{}); break;
+// Power of two by which block fixed-point transforms come out too small
+// (a factor 4 for every twiddled stage).
+template <int N> constexpr int fx_fft_shift = 2 * (FftPlan<N, FftE<fx64>::value>::NS - 1);
+
+// N-point transform of one FP64 row in block fixed point: inputs v in
+// FftIO::in_elem order, results in v in FftIO::out_elem order.  z: the size of
+// the row.  The caller has synchronised the row's threads since anything else
+// read or wrote its shared memory.
+template <int DIR, int N, bool WS, class Idx>
+__device__ __forceinline__ void fx_fft_regs(double2* s, const Idx& idx, int row, int t, bool act,
+                                            const longlong2* __restrict__ tw, int ts, FxSize z, double2* v) {
+    constexpr int EM = FftE<fx64>::value;
+    constexpr int K = FftPlan<N, EM>::E;
+    longlong2 o[K];
+    const FxExp x = fx_row<K, N == 512 ? 57 : 58, 62>(v, z, o);
+    smem_fft2<fx64, DIR, N, true, true, EM, WS>(reinterpret_cast<longlong2*>(s), idx, row, t, act, tw, ts, o);
+    fx_unrow<K>(o, x, fx_fft_shift<N>, v);
+}
+
+// The same for a column of a Z tile (column = thread % TZ): reads it from
+// the tile, leaves the results in v.  slot: see fx_column_size.
+template <int DIR, int N, int TZ, int NT, class Idx>
+__device__ __forceinline__ void fx_fft_column(double2* s, const Idx& idx, int c, int t,
+                                              const longlong2* __restrict__ tw, FxSlot* slot, double2* v) {
+    using IO = FftIO<fx64, DIR, N>;
+    FxSize z;
+#pragma unroll
+    for (int i = 0; i < IO::E; ++i) {
+        v[i] = s[idx(c, IO::in_elem(t, i))];
+        z.add(v[i]);
     }
+    z = fx_column_size<TZ, NT>(z, slot);
+    fx_fft_regs<DIR, N, false>(s, idx, c, t, true, tw, 1, z, v);
+}
+
+// Calls f(std::integral_constant<int, n>) for a power of two n in [LO, HI]
+// (axes are 8 to 512 long, rows along x half of that in complex pairs).
+template <int LO, int HI, class F> inline void dispatch_pow2(int n, F&& f) {
+    if constexpr (LO == HI) f(std::integral_constant<int, HI>{});
+    else if (n <= LO) f(std::integral_constant<int, LO>{});
+    else dispatch_pow2<2 * LO, HI>(n, f);
 }
 
 }  // namespace fipi

@@ -594,6 +594,22 @@ template <typename T> static fipi_status alloc_fields_t(fipi_ctx* ctx) {
     FIPI_CUDA(ctx, h2d(ctx, b.twx, tx.data(), sizeof(C) * g.nx));
     FIPI_CUDA(ctx, h2d(ctx, b.twy, ty.data(), sizeof(C) * g.ny));
     FIPI_CUDA(ctx, h2d(ctx, b.twz, tz.data(), sizeof(C) * g.nz));
+    if constexpr (sizeof(T) == sizeof(double)) {  // block fixed-point factors (fx64.cuh)
+        auto factors = [&](void** dst, int n) -> cudaError_t {
+            std::vector<longlong2> t(n);
+            const long double two_pi = 6.283185307179586476925286766559005768L, one = 4611686018427387904.0L;
+            for (int q = 0; q < n; ++q) {
+                const long double a = two_pi * (long double)q / (long double)n;
+                t[q].x = fx_pack(llrintl(cosl(a) * one));
+                t[q].y = fx_pack(llrintl(-sinl(a) * one));
+            }
+            const cudaError_t e = A(dst, sizeof(longlong2) * n);
+            return e != cudaSuccess ? e : h2d(ctx, *dst, t.data(), sizeof(longlong2) * n);
+        };
+        FIPI_CUDA(ctx, factors(&b.fwx, g.nx));
+        FIPI_CUDA(ctx, factors(&b.fwy, g.ny));
+        FIPI_CUDA(ctx, factors(&b.fwz, g.nz));
+    }
     // field.cpp:100-121: i*2.0*pi/L for i <= N/2 else (i - N)*2.0*pi/L
     const fipi_params& P = ctx->P;
     auto waves = [&](int n, int count, double L) {
@@ -634,7 +650,7 @@ fipi_status fields_alloc(fipi_ctx* ctx) {
 
 void fields_free(fipi_ctx* ctx) {
     FieldBufs& b = ctx->fb;
-    void* all[] = {b.twx, b.twy, b.twz, b.kx, b.ky, b.kz, b.c, b.ureal, b.chat, b.chat_old, b.fhat,
+    void* all[] = {b.twx, b.twy, b.twz, b.fwx, b.fwy, b.fwz, b.kx, b.ky, b.kz, b.c, b.ureal, b.chat, b.chat_old, b.fhat,
                    b.fhat_old, b.Chat_old, b.S[0], b.S[1], b.S[2], b.S[3], b.g[0], b.g[1], b.g[2],
                    b.fsp[0], b.fsp[1], b.fsp[2], b.upre[0], b.upre[1], b.upre[2], ctx->partials, ctx->k0};
     for (void* p : all)

@@ -348,6 +348,116 @@ __device__ __forceinline__ void r2c_post_regs(cplx<T>* s, const Idx& idx, int ro
     });
 }
 
+// The FP64 form's X rows in block fixed point (fx64.cuh), one row per Tn lanes
+// of a warp.  C2R: the row's M + 1 modes become integers in place, the
+// pre-processing (/ 4) feeds the inverse transform, and the M real pairs go
+// back to the tile as FP64 times 2^shift.  Every lane of the warp calls; act:
+// the lane's row exists.
+template <int M, class Idx>
+__device__ __forceinline__ void fx_c2r_row(double2* s, const Idx& idx, int row, int t, bool act,
+                                           const longlong2* __restrict__ tw, int shift) {
+    using PL = FftPlan<M, FftE<fx64>::value>;
+    using IO = FftIO<fx64, +1, M>;
+    constexpr int K = PL::E, Tn = PL::Tn;
+    constexpr int R0 = PL::radix(0, +1);
+    longlong2* si = reinterpret_cast<longlong2*>(s);
+    longlong2 o[K];
+    FxExp x;
+    {
+        double2 v[K + 1];
+#pragma unroll
+        for (int j = 0; j < K; ++j) v[j] = act ? s[idx(row, t + Tn * j)] : make_double2(0.0, 0.0);
+        v[K] = act && t == 0 ? s[idx(row, M)] : make_double2(0.0, 0.0);
+        if (t == 0) v[0].y = v[K].y = 0.0;  // only the real parts of X_0 and X_M enter
+        FxSize z;
+#pragma unroll
+        for (int j = 0; j <= K; ++j) z.add(v[j]);
+        z = fx_row_size<Tn>(z);
+        longlong2 w[K + 1];
+        x = fx_row<K + 1, 57, 61>(v, z, w);
+        if (act) {
+#pragma unroll
+            for (int j = 0; j < K; ++j) si[idx(row, t + Tn * j)] = w[j];
+            if (t == 0) si[idx(row, M)] = w[K];
+        }
+    }
+    __syncwarp();
+    static_for<0, K>([&](auto JC) {
+        constexpr int j = decltype(JC)::value;
+        const int k = t + Tn * j;
+        longlong2 z{};
+        if (act) {
+            const longlong2 xk = si[idx(row, k)], xm = si[idx(row, M - k)];
+            const longlong2 A = cadd(xk, cconj(xm)), B = csub(xk, cconj(xm));
+            z = cadd(fx_quarter(A), cmul_i(fx_mulw<+1>(B, tw[k]), +1));
+            if constexpr (j == 0)
+                if (t == 0) z = fx_quarter(mkc<longlong2>(xk.x + xm.x, xk.x - xm.x));
+        }
+        o[xslot_of_j<K, R0>(j)] = z;
+    });
+    __syncwarp();  // the row is read before the first stage writes it
+    smem_fft2<fx64, +1, M, true, true, FftE<fx64>::value, true>(si, idx, row, t, act, tw, 2, o);
+    double2 r[K];
+    fx_unrow<K>(o, x, shift + fx_fft_shift<M> + 2, r);
+    if (act)
+#pragma unroll
+        for (int i = 0; i < K; ++i) s[idx(row, IO::out_elem(t, i))] = r[i];
+}
+// R2C: M real pairs of the tile -> M + 1 modes in the tile (post-processing
+// / 2: X_k = (E - i W_k D) / 2 from quarters).
+template <int M, class Idx>
+__device__ __forceinline__ void fx_r2c_row(double2* s, const Idx& idx, int row, int t, bool act,
+                                           const longlong2* __restrict__ tw) {
+    using PL = FftPlan<M, FftE<fx64>::value>;
+    using IO = FftIO<fx64, -1, M>;
+    constexpr int K = PL::E, Tn = PL::Tn;
+    longlong2* si = reinterpret_cast<longlong2*>(s);
+    longlong2 o[K];
+    FxExp ex;
+    {
+        double2 v[K];
+        FxSize z;
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            v[i] = act ? s[idx(row, IO::in_elem(t, i))] : make_double2(0.0, 0.0);
+            z.add(v[i]);
+        }
+        z = fx_row_size<Tn>(z);
+        ex = fx_row<K, 57, 61>(v, z, o);
+    }
+    __syncwarp();
+    smem_fft2<fx64, -1, M, true, false, FftE<fx64>::value, true>(si, idx, row, t, act, tw, 2, o);
+    __syncwarp();
+    longlong2 zm0{};
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const int k = t + Tn * j;
+        longlong2 x{};
+        if (act) {
+            const longlong2 zk = si[idx(row, k)], zm = si[idx(row, (M - k) & (M - 1))];
+            const longlong2 Ev = cadd(zk, cconj(zm)), D = csub(zk, cconj(zm));
+            x = csub(fx_quarter(Ev), cmul_i(fx_mulw<-1>(D, tw[k]), +1));
+            if (k == 0) {
+                x = mkc<longlong2>((zk.x + zk.y + 1) >> 1, 0);
+                zm0 = mkc<longlong2>((zk.x - zk.y + 1) >> 1, 0);
+            }
+        }
+        o[j] = x;
+    }
+    __syncwarp();  // every mode is read before any is written
+    double2 r[K];
+    fx_unrow<K>(o, ex, fx_fft_shift<M> + 1, r);
+    if (act) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) s[idx(row, t + Tn * j)] = r[j];
+        if (t == 0) {
+            double2 xm;
+            fx_unrow<1>(&zm0, ex, fx_fft_shift<M> + 1, &xm);
+            s[idx(row, M)] = xm;
+        }
+    }
+}
+
 // X pass: one block = TY consecutive rows y0..y0+TY-1 of plane z, NIN
 // spectral inputs (transposed runs of TY along y, C2R) and NOUT spectral
 // outputs (R2C, transposed store); point() does the fused real-space work
@@ -386,8 +496,9 @@ struct HasRowPrefetch<O, std::void_t<decltype(std::declval<const O&>().prefetch_
 
 template <typename T, int NIN, int NOUT, bool REDUCE, int M, class Op, int NT = kThreads>
 __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), NT>::value)
-    k_xpass_acc(Geom g, const cplx<T>* __restrict__ twx, Op op, double* partials) {
+    k_xpass_acc(Geom g, const tw_t<T>* __restrict__ twx, Op op, double* partials) {
     using C = cplx<T>;
+    constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     constexpr int TY = x_rows<T, M>;
     constexpr int NF = NIN > NOUT ? NIN : NOUT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -403,7 +514,7 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     // field belongs to one warp from the split processing through the
     // point loop; the block synchronises only after each field's tile
     // load and before the tile stores
-    constexpr bool WL = kXWarpSync && TY * Tn == NT && M >= 32;
+    constexpr bool WL = !FX && kXWarpSync && TY * Tn == NT && M >= 32;
     // Loads and stores walk the tile field by field with ty fastest (a
     // run of TY along y per kx): each thread keeps one ty and steps kx.
     constexpr int KS = NT / TY;
@@ -423,7 +534,14 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
         }
         if constexpr (HasRowPrefetch<Op>::value)
             if (tid == 0) op.prefetch_rows(z, y0, TY);
-        if constexpr (WL) {
+        if constexpr (FX) {
+            cp_async_wait_all();
+            __syncthreads();
+            for (int r0 = 0; r0 < NIN * TY; r0 += rpr) {
+                const int row = r0 + tid / Tn;
+                fx_c2r_row<M>(s, idx, row, tid % Tn, row < NIN * TY, twx, -ilog2i(g.nx) - g.ly - g.lz);
+            }
+        } else if constexpr (WL) {
 #pragma unroll
             for (int f = 0; f < NIN; ++f) {
                 cp_async_wait_pending(NIN - 1 - f);
@@ -464,7 +582,10 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     auto point = [&](int ty, int n) {
         C v[NF];
 #pragma unroll
-        for (int f = 0; f < NIN; ++f) v[f] = cscale(s[idx(f * TY + ty, n)], invV);
+        for (int f = 0; f < NIN; ++f) {
+            if constexpr (FX) v[f] = s[idx(f * TY + ty, n)];  // 1/V is in the row's exponent
+            else v[f] = cscale(s[idx(f * TY + ty, n)], invV);
+        }
         op.point(z, y0 + ty, n, v, acc);
 #pragma unroll
         for (int f = 0; f < NOUT; ++f) s[idx(f * TY + ty, n)] = v[f];
@@ -488,7 +609,12 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     if constexpr (WL) __syncwarp();
     else __syncthreads();
     if constexpr (NOUT > 0) {
-        if constexpr (WL) {
+        if constexpr (FX) {
+            for (int r0 = 0; r0 < NOUT * TY; r0 += rpr) {
+                const int row = r0 + tid / Tn;
+                fx_r2c_row<M>(s, idx, row, tid % Tn, row < NOUT * TY, twx);
+            }
+        } else if constexpr (WL) {
 #pragma unroll
             for (int f = 0; f < NOUT; ++f) {
                 C v[EM];
@@ -726,7 +852,12 @@ template <typename T> struct F {
     static C* S(fipi_ctx* ctx, int i) { return (C*)ctx->fb.S[i]; }
     static C* sp(void* p) { return (C*)p; }
     static T* re(void* p) { return (T*)p; }
-    static const C* tw(void* p) { return (const C*)p; }
+    // the transforms' twiddle tables along x, y, z
+    static const tw_t<T>* tw(const fipi_ctx* ctx, int axis) {
+        const FieldBufs& b = ctx->fb;
+        constexpr bool fx = sizeof(T) == sizeof(double);
+        return (const tw_t<T>*)(axis == 0 ? (fx ? b.fwx : b.twx) : axis == 1 ? (fx ? b.fwy : b.twy) : (fx ? b.fwz : b.twz));
+    }
     static KTabs<T> ktabs(fipi_ctx* ctx) {
         return KTabs<T>{(const T*)ctx->fb.kx, (const T*)ctx->fb.ky, (const T*)ctx->fb.kz};
     }
@@ -740,7 +871,7 @@ void launch_x(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double* 
     LaunchScope ls(ctx, name,
                    (double)(NIN + NOUT) * g.SH * sizeof(cplx<T>) + (double)nreal * g.V * sizeof(T));
     constexpr int NF = NIN > NOUT ? NIN : NOUT;
-    dispatch_pow2(g.m, [&](auto MC) {
+    dispatch_pow2<4, 256>(g.m, [&](auto MC) {
         constexpr int M = decltype(MC)::value;
         constexpr int TY = x_rows<T, M>;
         const size_t smem = (size_t)NF * TY * xpass_pitch(g.m) * sizeof(cplx<T>);
@@ -748,7 +879,7 @@ void launch_x(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double* 
         auto kern = k_xpass_acc<T, NIN, NOUT, REDUCE, M, Op, NT>;
         static size_t granted = 48 * 1024;
         ensure_smem(kern, smem, granted);
-        kern<<<grid, NT, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twx, op, partials);
+        kern<<<grid, NT, smem, ctx->stream>>>(g, F<T>::tw(ctx, 0), op, partials);
     });
 }
 
@@ -764,7 +895,7 @@ void launch_xs(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double*
         LaunchScope ls(ctx, name,
                        (double)(NIN + NOUT) * g.SH * sizeof(cplx<T>) + (double)nreal * g.V * sizeof(T));
         constexpr int NF = NIN > NOUT ? NIN : NOUT;
-        dispatch_pow2(g.m, [&](auto MC) {
+        dispatch_pow2<4, 256>(g.m, [&](auto MC) {
             constexpr int M = decltype(MC)::value;
             constexpr int TY = x_rows<T, M>;
             const size_t smem = (size_t)NF * TY * xpass_pitch(g.m) * sizeof(cplx<T>);
@@ -773,13 +904,13 @@ void launch_xs(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double*
                 auto kern = k_xpass_stream<T, NIN, NOUT, REDUCE, M, Op>;
                 static size_t granted = 48 * 1024;
                 ensure_smem(kern, smem, granted);
-                kern<<<grid, XStreamShape<T, M>::NT, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twx, op,
+                kern<<<grid, XStreamShape<T, M>::NT, smem, ctx->stream>>>(g, F<T>::tw(ctx, 0), op,
                                                                             partials);
             } else {  // rows of more than 256 points: one round per field would need > 256 threads
                 auto kern = k_xpass_acc<T, NIN, NOUT, REDUCE, M, Op>;
                 static size_t granted = 48 * 1024;
                 ensure_smem(kern, smem, granted);
-                kern<<<grid, kThreads, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twx, op, partials);
+                kern<<<grid, kThreads, smem, ctx->stream>>>(g, F<T>::tw(ctx, 0), op, partials);
             }
         });
     }
@@ -797,7 +928,7 @@ template <typename T> void launch_y(fipi_ctx* ctx, int nf, void* const* in, void
     }
     // persistent, TMA double-buffered: a grid of resident blocks walks all tiles
     const size_t smem = ypass_tma_smem<T>(g);
-    dispatch_pow2(g.ny, [&](auto NC) {
+    dispatch_pow2<8, 512>(g.ny, [&](auto NC) {
         constexpr int N = decltype(NC)::value;
         auto kern = (dir < 0) ? k_ypass_tma<T, -1, N> : k_ypass_tma<T, +1, N>;
         static size_t granted[2] = {48 * 1024, 48 * 1024};
@@ -812,7 +943,7 @@ template <typename T> void launch_y(fipi_ctx* ctx, int nf, void* const* in, void
         const long long tiles = ((long long)g.nz * g.h + rb - 1) / rb * nf;
         long long grid = (long long)ctx->num_sms * blocks_per_sm[di];
         if (grid > tiles) grid = tiles;
-        kern<<<(unsigned)grid, kThreads, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twy, fp, nf, ctx->status,
+        kern<<<(unsigned)grid, kThreads, smem, ctx->stream>>>(g, F<T>::tw(ctx, 1), fp, nf, ctx->status,
                                                               ctx->debug_first_wait);
     });
 }
@@ -824,12 +955,12 @@ template <typename T, int NF, int DIR, class Op> void launch_z(fipi_ctx* ctx, co
     const size_t smem = zpass_smem<T, NF>(g);
     dim3 grid(g.h, g.ny / zpass_cols<T>(g.nz));
     const int threads = zpass_threads<T>(g.nz);
-    dispatch_pow2(g.nz, [&](auto NC) {
+    dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
         constexpr int N = decltype(NC)::value;
         auto kern = k_zpass<T, NF, DIR, N, Op>;
         static size_t granted = 48 * 1024;
         ensure_smem(kern, smem, granted);
-        kern<<<grid, threads, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twz, op);
+        kern<<<grid, threads, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
     });
 }
 
@@ -851,7 +982,7 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
     constexpr int EM = zrt_elems<T, NF, NB>;
     if constexpr (sizeof(T) == sizeof(float) && zrt_in_registers<NF, NB>) {
         // FP32: the round trip held in registers
-        dispatch_pow2(g.nz, [&](auto NC) {
+        dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
             constexpr int N = decltype(NC)::value;
             using SHP = ZRtShapeT<T, N, 16, EM>;
             const size_t smem = (size_t)(HasAux<Op>::value ? 2 : 1) * SHP::TZ * N * sizeof(cplx<T>);
@@ -859,12 +990,12 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
             auto kern = k_zpass_rr<T, NF, NB, DIR, N, 16, Op, EM>;
             static size_t granted = 48 * 1024;
             ensure_smem(kern, smem, granted);
-            kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twz, op);
+            kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
         });
         return;
     }
     if constexpr (!WIDE) {
-        dispatch_pow2(g.nz, [&](auto NC) {
+        dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
             constexpr int N = decltype(NC)::value;
             using SHP = ZRtShapeT<T, N, COLS, EM>;
             constexpr int NS = NF > NB ? NF : NB;
@@ -873,11 +1004,11 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
             auto kern = k_zpass_rt_t<T, NF, NB, DIR, N, COLS, Op, EM>;
             static size_t granted = 48 * 1024;
             ensure_smem(kern, smem, granted);
-            kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twz, op);
+            kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
         });
         return;
     } else
-    dispatch_pow2(g.nz, [&](auto NC) {
+    dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
         constexpr int N = decltype(NC)::value;
         constexpr int NS = NF > NB ? NF : NB;
         // columns of 512 modes with three or more fields: half the tile (two blocks per SM)
@@ -888,7 +1019,7 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
         auto kern = k_zpass_rt<T, NF, NB, DIR, N, CW, Op, EM>;
         static size_t granted = 48 * 1024;
         ensure_smem(kern, smem, granted);
-        kern<<<grid, SHP::THREADS, smem, ctx->stream>>>(g, (const cplx<T>*)ctx->fb.twz, op);
+        kern<<<grid, SHP::THREADS, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
     });
 }
 
