@@ -373,18 +373,19 @@ template <typename T, int N, int COLS, int EM = FftE<T>::value> struct ZRtShape 
     static constexpr int RC = COLS * Tn <= kThreads ? COLS : kThreads / Tn;  // columns per FFT round
     static constexpr int THREADS = RC * Tn;
     static constexpr int P = COLS + 1;  // shared-memory pitch of one kz row (odd: fewer bank conflicts)
-    // WZ (FP32, one round of column FFTs of at most a warp each): the
-    // forward transforms and the first stage of each inverse run on columns
-    // owned by single warps; the tile then adds one pad slot per 16 kz rows
-    // so that the strided writes of a column's first stage meet no bank
-    // conflicts
-    static constexpr bool WZ = sizeof(T) == 4 && RC == COLS && Tn <= 32 && FftPlan<N, EM>::NS >= 2;
-    static constexpr int FSTRIDE = N * P + (WZ ? N / 16 : 0);  // complex entries per field tile
+    // WZ (one round of column FFTs of at most a warp each): the forward
+    // transforms and the first stage of each inverse (FP64: all of it) run on
+    // columns owned by single warps; the tile then adds one pad slot per 2^PAD
+    // kz rows so that the strided writes of a column's first stage meet no
+    // bank conflicts
+    static constexpr bool WZ = RC == COLS && Tn <= 32 && THREADS >= 32 && FftPlan<N, EM>::NS >= 2;
+    static constexpr int PAD = !WZ ? 0 : sizeof(T) == 4 ? 4 : 3;
+    static constexpr int FSTRIDE = N * P + (PAD ? N >> PAD : 0);  // complex entries per field tile
 };
-// Z round-trip tile index: mode e of column c, with the WZ pad slots.
-template <bool PAD> struct IdxZ {
+// Z round-trip tile index: mode e of column c, with the pad slots.
+template <int PAD> struct IdxZ {
     int cols;
-    __device__ __forceinline__ int operator()(int c, int e) const { return e * cols + c + (PAD ? (e >> 4) : 0); }
+    __device__ __forceinline__ int operator()(int c, int e) const { return e * cols + c + (PAD ? (e >> PAD) : 0); }
 };
 
 // The tile is COLS columns (a 128-byte run of ky per kz for FP32 and FP64)
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __
     const size_t zstride = (size_t)g.h * g.ny;
     const size_t base = (size_t)kx * g.ny + ky0;
     constexpr bool WZ = SH::WZ;
-    const IdxZ<WZ> idx{P};
+    const IdxZ<SH::PAD> idx{P};
     constexpr size_t fstride = SH::FSTRIDE;
     op.prologue();
     if constexpr (HasSrc<Op>::value) {
@@ -445,7 +446,13 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __
             cp_async_wait_pending(NF - 1 - f);
             __syncthreads();
         }
-        if constexpr (WZ) smem_fft2<T, DIR, N, EM, true>(s + f * fstride, idx, wc, wt, true, twz, 1);
+        if constexpr (WZ && FX) {
+            C v[SH::E];
+            fx_fft_warp_column<DIR, N>(s + f * fstride, idx, wc, wt, twz, v);
+            using IOF = FftIO<T, DIR, N, EM>;
+#pragma unroll
+            for (int i = 0; i < SH::E; ++i) s[f * fstride + idx(wc, IOF::out_elem(wt, i))] = v[i];
+        } else if constexpr (WZ) smem_fft2<T, DIR, N, EM, true>(s + f * fstride, idx, wc, wt, true, twz, 1);
         else
             for (int r = 0; r < COLS; r += RC) {
                 if constexpr (FX) {
@@ -499,6 +506,24 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __
     // slot a warp writes RC consecutive columns of Tn-strided modes (full
     // 128-byte runs), field by field while the next field is transformed
     using IO = FftIO<T, -DIR, N, EM>;
+    if constexpr (WZ && FX) {
+        // FP64: whole inverse transforms on the warps' columns, then full runs
+        // from the tile
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            C v[SH::E];
+            fx_fft_warp_column<-DIR, N>(s + b * fstride, idx, wc, wt, twz, v);
+#pragma unroll
+            for (int i = 0; i < SH::E; ++i) s[b * fstride + idx(wc, IO::out_elem(wt, i))] = v[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            for (int e = tid; e < ELEMS; e += NT) {
+                const int c = e % COLS, z = e / COLS;
+                op.rr_store(b, base + c + z * zstride, s[b * fstride + idx(c, z)]);
+            }
+    } else {
 #pragma unroll
     for (int b = 0; b < NB; ++b)
         for (int r = 0; r < COLS; r += RC) {
@@ -516,6 +541,7 @@ __global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __
 #pragma unroll
             for (int i = 0; i < SH::E; ++i) op.rr_store(b, base + r + cl + (size_t)IO::out_elem(t, i) * zstride, v[i]);
         }
+    }
 }
 
 // Round trip with the column-per-thread-group mapping of k_zpass: the tile
@@ -696,6 +722,70 @@ __global__ void __launch_bounds__(kThreads, 2) k_zpass_rr(Geom g, const tw_t<T>*
         for (int i = 0; i < E; ++i) {
             const int z = IOI::out_elem(t, i);
             op.rr_store(b, base + z * zstride, v[i]);
+        }
+    }
+}
+
+// The FP64 counterpart of k_zpass_rr: one input whose transform feeds NB
+// outputs formed one at a time from it and a staged aux array.  Columns are
+// owned by warps (ZRtShape's WZ), so the transforms take no block barrier;
+// the tile of the input carries every output to its coalesced store in turn,
+// the aux tile stays.  Two tiles instead of NB (the earlier form, k_zpass_rt_t
+// with 4-column tiles of all four outputs: one SM held 12 warps): ZRRT.
+template <int NB, int DIR, int N, int COLS, class Op>
+__global__ void __launch_bounds__(kThreads, 2) k_zpass_rr_fx(Geom g, const longlong2* __restrict__ twz, Op op) {
+    using C = double2;
+    using SH = ZRtShape<double, N, COLS>;
+    constexpr int NT = SH::THREADS, ELEMS = COLS * N, E = SH::E, Tn = SH::Tn;
+    using IOF = FftIO<double, DIR, N>;
+    using IOI = FftIO<double, -DIR, N>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* s = reinterpret_cast<C*>(smem_raw);
+    C* sa = s + SH::FSTRIDE;
+    const IdxZ<SH::PAD> idx{SH::P};
+    const int kx = blockIdx.x, ky0 = blockIdx.y * COLS;
+    const int tid = threadIdx.x, wc = tid / Tn, wt = tid % Tn;
+    const size_t zstride = (size_t)g.h * g.ny;
+    const size_t base = (size_t)kx * g.ny + ky0;
+    for (int e = tid; e < ELEMS; e += NT) cp_async<16>(&s[idx(e % COLS, e / COLS)], op.src(0) + base + e % COLS + (e / COLS) * zstride);
+    cp_async_commit();
+    for (int e = tid; e < ELEMS; e += NT) cp_async<16>(&sa[idx(e % COLS, e / COLS)], op.aux() + base + e % COLS + (e / COLS) * zstride);
+    cp_async_commit();
+    cp_async_wait_pending(1);
+    __syncthreads();
+    C v[E];
+    fx_fft_warp_column<DIR, N>(s, idx, wc, wt, twz, v);
+#pragma unroll
+    for (int i = 0; i < E; ++i) s[idx(wc, IOF::out_elem(wt, i))] = v[i];
+    cp_async_wait_all();
+    __syncthreads();
+    for (int e = tid; e < ELEMS; e += NT) {
+        const int c = e % COLS, z = e / COLS;
+        typename Op::State st;
+        const C w = s[idx(c, z)];
+        op.rr_mid(kx, ky0 + c, z, base + c + z * zstride, &w, sa[idx(c, z)], st);  // stores the input's spectrum
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        FxSize size;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const int z = IOF::out_elem(wt, i);
+            typename Op::State st;
+            if (b == 0) st.f = v[i];
+            v[i] = op.rr_out(b, kx, ky0 + wc, z, st, sa[idx(wc, z)]);
+            size.add(v[i]);
+        }
+        size = fx_row_size<Tn>(size);
+        __syncthreads();  // the tile's previous contents are stored
+        fx_fft_regs<-DIR, N, true>(s, idx, wc, wt, true, twz, 1, size, v);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < E; ++i) s[idx(wc, IOI::out_elem(wt, i))] = v[i];
+        __syncthreads();
+        for (int e = tid; e < ELEMS; e += NT) {
+            const int c = e % COLS, z = e / COLS;
+            op.rr_store(b, base + c + z * zstride, s[idx(c, z)]);
         }
     }
 }

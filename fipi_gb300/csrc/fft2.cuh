@@ -295,6 +295,23 @@ __device__ __forceinline__ void fx_fft_column(double2* s, const Idx& idx, int c,
     fx_fft_regs<DIR, N, false>(s, idx, c, t, true, tw, 1, z, v);
 }
 
+// The same for a column whose Tn threads are consecutive lanes of one warp
+// (no block barrier).
+template <int DIR, int N, class Idx>
+__device__ __forceinline__ void fx_fft_warp_column(double2* s, const Idx& idx, int c, int t,
+                                                   const longlong2* __restrict__ tw, double2* v) {
+    using IO = FftIO<fx64, DIR, N>;
+    FxSize z;
+#pragma unroll
+    for (int i = 0; i < IO::E; ++i) {
+        v[i] = s[idx(c, IO::in_elem(t, i))];
+        z.add(v[i]);
+    }
+    z = fx_row_size<IO::PL::Tn>(z);
+    __syncwarp();  // the column is read before the first stage writes it
+    fx_fft_regs<DIR, N, true>(s, idx, c, t, true, tw, 1, z, v);
+}
+
 // Calls f(std::integral_constant<int, n>) for a power of two n in [LO, HI]
 // (axes are 8 to 512 long, rows along x half of that in complex pairs).
 template <int LO, int HI, class F> inline void dispatch_pow2(int n, F&& f) {

@@ -182,7 +182,14 @@ template <typename T> struct OpForce {
         // buoyancy ((1+c)/2 rho1 + (1-c)/2 rho2) g, g = (0, 0, gravity); with
         // gravity = 0 it adds exactly zero and c is not read
         T b0 = T(0), b1 = T(0);
-        if (gravity != T(0)) {
+        if (sizeof(T) == sizeof(double) && gravity != T(0)) {
+            // FP64: gravity (rho1 + rho2)/2 + c gravity (rho1 - rho2)/2, one
+            // instruction a point (gravity is applied here)
+            const C cc = r.get(0, n);
+            const T w0 = gravity * (rho1 + rho2) * T(0.5), w1 = gravity * (rho1 - rho2) * T(0.5);
+            b0 = cc.x * w1 + w0;
+            b1 = cc.y * w1 + w0;
+        } else if (gravity != T(0)) {
             const C cc = r.get(0, n);
             b0 = ((cc.x + T(1)) / T(2)) * rho1 + ((cc.x * T(-1) + T(1)) / T(2)) * rho2;
             b1 = ((cc.y + T(1)) / T(2)) * rho1 + ((cc.y * T(-1) + T(1)) / T(2)) * rho2;
@@ -197,7 +204,10 @@ template <typename T> struct OpForce {
                 f0 += sp.x;
                 f1 += sp.y;
             }
-            if (d == 2 && gravity != T(0)) {
+            if (d == 2 && sizeof(T) == sizeof(double)) {
+                f0 += b0;
+                f1 += b1;
+            } else if (d == 2 && gravity != T(0)) {
                 f0 += b0 * gravity;
                 f1 += b1 * gravity;
             }
@@ -280,8 +290,8 @@ template <typename T, bool MIXED> struct ZOpCH {
             im -= Cn.y * k.s4c;
             re += Co.x * k.s2c;
             im += Co.y * k.s2c;
-            const T den = k4 * k.s3 + T(3);
-            out = mkc<C>(re / den, im / den);
+            const T r = fast_inv(k4 * k.s3 + T(3));
+            out = mkc<C>(re * r, im * r);
         } else {
             const T a4 = k2 * k.s4;
             T re = c.x * T(4) + p.Co.x, im = c.y * T(4) + p.Co.y;
@@ -897,7 +907,7 @@ template <typename T> static void step_stokes_t(fipi_ctx* ctx) {
     launch_x<T, 4, 3, false>(ctx, "X inverse mu,grad, force, forward", nreal, of);
     void* s3[3] = {b.S[0], b.S[1], b.S[2]};
     launch_y<T>(ctx, 3, s3, s3, -1);
-    ZOpProj<T> zp{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, {nullptr, nullptr, nullptr}, kt, k.mu, g.m,
+    ZOpProj<T> zp{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, {nullptr, nullptr, nullptr}, kt, k.mu, T(1.0 / ctx->P.mu), g.m,
                   g.ny / 2, g.nz / 2};
     ZOpProjRt<T> zpr{zp, {F<T>::sp(b.upre[0]), F<T>::sp(b.upre[1]), F<T>::sp(b.upre[2])}};
     launch_zrt<T, 3, 3, -1, 16 / (sizeof(T) / 4), true>(ctx, "Z forward + projection + inverse", 6, zpr);
@@ -1060,7 +1070,7 @@ template <typename T> static fipi_status div_t(fipi_ctx* ctx, const double* v, d
     launch_y<T>(ctx, 3, s3, s3, -1);
     ZOpDivRt<T> zd{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, F<T>::S(ctx, 3), F<T>::ktabs(ctx), g.m,
                    g.ny / 2, g.nz / 2};
-    launch_zrt<T, 3, 1, -1, 16 / (sizeof(T) / 4), false>(ctx, "Z forward + div + inverse", 4, zd);
+    launch_zrt<T, 3, 1, -1, 16 / (sizeof(T) / 4), sizeof(T) == sizeof(double)>(ctx, "Z forward + div + inverse", 4, zd);
     void* s1[1] = {ctx->fb.S[3]};
     launch_y<T>(ctx, 1, s1, s1, +1);
     OpC2RStore<T, 1> oc{{F<T>::S(ctx, 3)}, {tmp}, g.nx, g.ny};

@@ -142,18 +142,16 @@ __device__ __forceinline__ long long fx_from(double x, int E, int B) {
     const long long r = (long long)(m >> s), sg = (long long)(hi >> 31);
     return (r ^ sg) - sg;
 }
-// a 2^q, rounded to nearest.
+// a 2^q, rounded to nearest (the rounding carry runs into the exponent field).
 __device__ __forceinline__ double fx_to(long long a, int q) {
     const int sg = fx_hi(a) & 0x80000000;
     const unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
-    const int z = __clzll((long long)u);
-    const unsigned long long m = (u << z) + 0x400ull;  // leading one at bit 63, half a unit added
-    const int c = m < 0x400ull;                        // carried out: 2^64
-    const int e = q + 1086 - z + c;                    // 1023 + 63
-    if (u == 0 || (unsigned)(e - 1) >= 2046u)          // zero, or outside the normal range
-        return u == 0 || e < 1 ? 0.0 : __hiloint2double(sg | 0x7ff00000, 0);
-    const unsigned long long f = m >> 11;              // bit 52: the leading one (0 after a carry)
-    return __hiloint2double((int)((unsigned)(f >> 32) & 0xfffffu) | (e << 20) | sg, (int)(unsigned)f);
+    const int z = __clzll((long long)u);  // >= 1: |a| < 2^63
+    const unsigned long long r = ((u << (z - 1)) + 0x200ull) >> 10;  // leading one at bit 52
+    const int e = q + 1085 - z;  // exponent field less one (1023 + 63)
+    if (u == 0 || (unsigned)e >= 2045u)  // zero, or outside the normal range
+        return u == 0 || e < 0 ? 0.0 : __hiloint2double(sg | 0x7ff00000, 0);
+    return __hiloint2double(((int)(r >> 32) + (e << 20)) | sg, (int)(unsigned)r);
 }
 __device__ __forceinline__ double2 fx_to(longlong2 a, int q) {
     double2 o;

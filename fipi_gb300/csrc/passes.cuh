@@ -64,6 +64,21 @@ template <typename T> struct KTabs {
     }
 };
 
+// 1/x in FP64 from an FP32 estimate (converted both ways on the bits; a
+// conversion or a division runs on the FP64 pipe, which issues at 1/64 of the
+// FP32 rate) and one third-order step r (1 + e + e^2), e = 1 - x r, |e| <
+// 2^-20: three FP64 instructions, within 1.5 units in the last place.  x
+// outside (2^-126, 2^126), negative or NaN: the division.
+__device__ __forceinline__ double fast_inv(double x) {
+    const int h = __double2hiint(x);
+    if ((unsigned)(h - ((1023 - 126) << 20)) >= (252u << 20)) return 1.0 / x;
+    const float r0 = __fdividef(1.f, __int_as_float(((h - (896 << 20)) << 3) | (int)((unsigned)__double2loint(x) >> 29)));
+    const int b = __float_as_int(r0);
+    const double r = __hiloint2double((b >> 3) + (896 << 20), b << 29);
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // ------------------------------------------------------------ block reduce
 __device__ __forceinline__ double block_sum(double v) {
     __shared__ double red[32];
@@ -485,7 +500,18 @@ constexpr bool kXWarpSync = true;
 template <typename T, int NIN, int NOUT> constexpr int x_elems = FftE<T>::value;
 
 template <typename T, int NF, int NT> struct XMinBlocks {
-    static constexpr int value = sizeof(T) == 4 ? (NF <= 3 ? 4 : 3) : (NF <= 3 ? 3 : 2);
+    static constexpr int value = NF <= 3 ? 4 : 3;
+};
+// FP64 (block fixed point): for rows of 32 to 256 pairs the block is one field's
+// rows, so each row of every field belongs to one warp from the conversion to
+// the last (no idle lanes for an odd number of fields, no block barrier between
+// the transforms and the point loop); shorter rows share 256 threads.  The
+// register budget follows what the tile leaves room for.  Against 256
+// threads with block-wide rounds: XFXT.
+template <int M> constexpr int x_fx_threads = M >= 32 ? x_rows_of(8, M) * FftPlan<M, 8>::Tn : kThreads;
+template <int NF, int NT> struct XMinBlocks<double, NF, NT> {
+    static constexpr int at128 = NF <= 2 ? 6 : NF == 3 ? 4 : NF == 4 ? 3 : 2;
+    static constexpr int value = at128 * 128 / NT > 0 ? at128 * 128 / NT : 1;
 };
 
 // op.prefetch_rows(z, y0, rows): L2 prefetches of the real rows the point
@@ -514,7 +540,8 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     // field belongs to one warp from the split processing through the
     // point loop; the block synchronises only after each field's tile
     // load and before the tile stores
-    constexpr bool WL = !FX && kXWarpSync && TY * Tn == NT && M >= 32;
+    // (FP64: also no barrier between a field's load and the next)
+    constexpr bool WL = kXWarpSync && TY * Tn == NT && M >= 32;
     // Loads and stores walk the tile field by field with ty fastest (a
     // run of TY along y per kx): each thread keeps one ty and steps kx.
     constexpr int KS = NT / TY;
@@ -522,7 +549,7 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     const size_t gbase = (size_t)z * H * g.ny + y0 + tyl;
     const int rrow = tid / Tn, rt = tid % Tn;  // WL: the row of a field this thread transforms
     C Wt{};
-    if constexpr (WL) Wt = twx[rt];
+    if constexpr (WL && !FX) Wt = twx[rt];
     if constexpr (NIN > 0) {
         // every element of the tile is requested before any is waited for,
         // one cp.async group per field
@@ -534,7 +561,15 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
         }
         if constexpr (HasRowPrefetch<Op>::value)
             if (tid == 0) op.prefetch_rows(z, y0, TY);
-        if constexpr (FX) {
+        if constexpr (FX && WL) {
+#pragma unroll 1
+            for (int f = 0; f < NIN; ++f) {
+                cp_async_wait_pending(NIN - 1 - f);
+                __syncthreads();
+                fx_c2r_row<M>(s, idx, f * TY + rrow, rt, true, twx, -ilog2i(g.nx) - g.ly - g.lz);
+            }
+            __syncwarp();
+        } else if constexpr (FX) {
             cp_async_wait_all();
             __syncthreads();
             for (int r0 = 0; r0 < NIN * TY; r0 += rpr) {
@@ -609,7 +644,10 @@ __global__ void __launch_bounds__(NT, XMinBlocks<T, (NIN > NOUT ? NIN : NOUT), N
     if constexpr (WL) __syncwarp();
     else __syncthreads();
     if constexpr (NOUT > 0) {
-        if constexpr (FX) {
+        if constexpr (FX && WL) {
+#pragma unroll 1
+            for (int f = 0; f < NOUT; ++f) fx_r2c_row<M>(s, idx, f * TY + rrow, rt, true, twx);
+        } else if constexpr (FX) {
             for (int r0 = 0; r0 < NOUT * TY; r0 += rpr) {
                 const int row = r0 + tid / Tn;
                 fx_r2c_row<M>(s, idx, row, tid % Tn, row < NOUT * TY, twx);
@@ -762,14 +800,14 @@ template <typename T> struct ZOpProj {
     C* out[3];
     __device__ const C* src(int f) const { return in[f]; }
     KTabs<T> kt;
-    T mu;
+    T mu, inv_mu;
     int m, ny2, nz2;
     __device__ void load(int, int, int, size_t gi, C* v) const {
         v[0] = in[0][gi];
         v[1] = in[1][gi];
         v[2] = in[2][gi];
     }
-    __device__ static void project(const T* kv, T k2, T mk2, const C* F, C* u) {
+    __device__ void project(const T* kv, T k2, T mk2, const C* F, C* u) const {
         T dre = T(0), dim = T(0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -785,12 +823,13 @@ template <typename T> struct ZOpProj {
                 u[d] = mkc<C>((F[d].x - qre) * r2, (F[d].y - qim) * r2);
             }
         } else {
-            // FP64: the reference's evaluation order (main.cpp:177-178)
+            // FP64: (F - k (k.F)/k^2) / (mu k^2) with one reciprocal instead of
+            // twelve divisions (PROJT)
+            const T r1 = fast_inv(k2), r2 = r1 * inv_mu;
+            dre *= r1;
+            dim *= r1;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const T qre = (kv[d] * dre) / k2, qim = (kv[d] * dim) / k2;
-                u[d] = mkc<C>((F[d].x - qre) / mk2, (F[d].y - qim) / mk2);
-            }
+            for (int d = 0; d < 3; ++d) u[d] = mkc<C>(fma(-kv[d], dre, F[d].x) * r2, fma(-kv[d], dim, F[d].y) * r2);
         }
     }
     __device__ void store(int ix, int iy, int iz, size_t gi, const C* F) const {
@@ -864,8 +903,8 @@ template <typename T> struct F {
 };
 
 // nreal: real (V-sized) arrays the fused point operation reads or writes.
-// One block per tile of x_rows<T, M> rows; NT threads per block.
-template <typename T, int NIN, int NOUT, bool REDUCE, class Op, int NT = kThreads>
+// One block per tile of x_rows<T, M> rows.
+template <typename T, int NIN, int NOUT, bool REDUCE, class Op>
 void launch_x(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double* partials = nullptr) {
     const Geom& g = ctx->g;
     LaunchScope ls(ctx, name,
@@ -874,6 +913,7 @@ void launch_x(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double* 
     dispatch_pow2<4, 256>(g.m, [&](auto MC) {
         constexpr int M = decltype(MC)::value;
         constexpr int TY = x_rows<T, M>;
+        constexpr int NT = sizeof(T) == sizeof(double) ? x_fx_threads<M> : kThreads;
         const size_t smem = (size_t)NF * TY * xpass_pitch(g.m) * sizeof(cplx<T>);
         dim3 grid(g.ny / TY, g.nz);
         auto kern = k_xpass_acc<T, NIN, NOUT, REDUCE, M, Op, NT>;
@@ -997,14 +1037,24 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
     if constexpr (!WIDE) {
         dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
             constexpr int N = decltype(NC)::value;
-            using SHP = ZRtShapeT<T, N, COLS, EM>;
-            constexpr int NS = NF > NB ? NF : NB;
-            const size_t smem = (size_t)NS * SHP::TZ * N * sizeof(cplx<T>);
-            dim3 grid(g.h, g.ny / SHP::TZ);
-            auto kern = k_zpass_rt_t<T, NF, NB, DIR, N, COLS, Op, EM>;
-            static size_t granted = 48 * 1024;
-            ensure_smem(kern, smem, granted);
-            kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
+            if constexpr (sizeof(T) == sizeof(double) && HasAux<Op>::value && ZRtShape<T, N, 2 * COLS>::WZ) {
+                // FP64 columns of 32 to 256 modes (at most a warp each)
+                using SHF = ZRtShape<T, N, 2 * COLS>;
+                const size_t smem = 2 * SHF::FSTRIDE * sizeof(cplx<T>);
+                auto kern = k_zpass_rr_fx<NB, DIR, N, 2 * COLS, Op>;
+                static size_t granted = 48 * 1024;
+                ensure_smem(kern, smem, granted);
+                kern<<<dim3(g.h, g.ny / (2 * COLS)), SHF::THREADS, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
+            } else {
+                using SHP = ZRtShapeT<T, N, COLS, EM>;
+                constexpr int NS = NF > NB ? NF : NB;
+                const size_t smem = (size_t)NS * SHP::TZ * N * sizeof(cplx<T>);
+                dim3 grid(g.h, g.ny / SHP::TZ);
+                auto kern = k_zpass_rt_t<T, NF, NB, DIR, N, COLS, Op, EM>;
+                static size_t granted = 48 * 1024;
+                ensure_smem(kern, smem, granted);
+                kern<<<grid, SHP::TZ * SHP::Tn, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
+            }
         });
         return;
     } else

@@ -84,8 +84,7 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) 
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Waits until at most n of this thread's committed groups are pending
-// (n folds to a constant where the caller's loop is unrolled; n > 3 waits
-// as for 3).
+// (n > 3 waits as for 3).
 __device__ __forceinline__ void cp_async_wait_pending(int n) {
     switch (n) {
         case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
