@@ -76,7 +76,6 @@ struct ParticleBufs {
     // diagnostics
     double* tau_part = nullptr;  // n, per-particle packing-energy terms
     float4* spos = nullptr;      // n, sorted cell-relative FP32 positions + id
-    int4* ipos = nullptr;        // n, positions as 32-bit fractions of the box (mixed form)
     void* sp_fw = nullptr;       // 6 x n (TA): spread force density (3) and trilinear fractions (3)
     unsigned long long* ymax = nullptr;  // [max p_y bits, first index] for it_mark
     bool tau_valid = false;

@@ -99,8 +99,9 @@ template <typename T> __host__ __device__ inline int ypass_rows(int ny) {
 // tile, the last stage stores straight to global memory.  `fields` fields of
 // rows are processed in one launch.
 constexpr int kYStages = 2;  // 3 measured no faster on GB300 (more registers)
-// FP32: three blocks per SM (<= 85 registers) measured 6 % faster than two
-// with the radix-16 codelets; FP64 keeps two (its codelets need ~124).
+// Three blocks per SM (<= 85 registers): FP32 (radix-16 codelets) 6 % faster
+// than two, FP64 (block fixed point; 128 registers with two) 304 -> 275 us for
+// three fields of 256^3.
 // FFT rounds per Y tile (one: 16 FP32 or 8 FP64 rows of 256, 32 KB per copy).
 template <typename T> struct YGroups {
     static constexpr int value = 1;
@@ -109,7 +110,7 @@ template <typename T> struct YGroups {
 // first_wait: polls of the block's first copy wait (-1: the normal bound);
 // a test hook that lets the bounded-wait error path run (fipi_set_debug).
 template <typename T, int DIR, int N>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_ypass_tma(Geom g, const tw_t<T>* __restrict__ twy, FieldPtrs<T> fp,
+__global__ void __launch_bounds__(kThreads, 3) k_ypass_tma(Geom g, const tw_t<T>* __restrict__ twy, FieldPtrs<T> fp,
                                                        int fields, int* status, int first_wait) {
     using C = cplx<T>;
     constexpr int EM = YE<T>::value;
@@ -392,8 +393,11 @@ template <int PAD> struct IdxZ {
 // of all kz; the column FFTs run in rounds of RC columns, while loads and
 // the mid operation walk the tile with ky fastest (full runs per warp).
 // Tiles whose load() only copies arrays (src()) arrive by cp.async.
+// Blocks per SM: four with one field (FP64: three, CH update 526 -> 450 us at
+// 256^3), two with three (their tiles take 105 KB and
+// 112 KB; FP32 projection at 512^3 2268 -> 1990 us against no bound).
 template <typename T, int NF, int NB, int DIR, int N, int COLS, class Op, int EM = FftE<T>::value>
-__global__ void __launch_bounds__(kThreads) k_zpass_rt(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(kThreads, NF == 1 && NB == 1 ? (sizeof(T) == 4 ? 4 : 3) : 2) k_zpass_rt(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
     constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     using SH = ZRtShape<T, N, COLS, EM>;
@@ -731,9 +735,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_zpass_rr(Geom g, const tw_t<T>*
 // owned by warps (ZRtShape's WZ), so the transforms take no block barrier;
 // the tile of the input carries every output to its coalesced store in turn,
 // the aux tile stays.  Two tiles instead of NB (the earlier form, k_zpass_rt_t
-// with 4-column tiles of all four outputs: one SM held 12 warps): ZRRT.
+// with 4-column tiles of all four outputs, 12 warps on an SM): 1261 -> 936 us at
+// 256^3 (three blocks of 85 registers an SM; 979 with two of 128).
 template <int NB, int DIR, int N, int COLS, class Op>
-__global__ void __launch_bounds__(kThreads, 2) k_zpass_rr_fx(Geom g, const longlong2* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(ZRtShape<double, N, COLS>::THREADS, ZRtShape<double, N, COLS>::THREADS == kThreads ? 3 : 512 / ZRtShape<double, N, COLS>::THREADS)
+    k_zpass_rr_fx(Geom g, const longlong2* __restrict__ twz, Op op) {
     using C = double2;
     using SH = ZRtShape<double, N, COLS>;
     constexpr int NT = SH::THREADS, ELEMS = COLS * N, E = SH::E, Tn = SH::Tn;

@@ -59,8 +59,7 @@ struct PC {
     double drag;       // 6 pi mu: the Stokes drag is drag * r
     double img[3];     // d_cell (n_cell - 2): the minimum-image threshold
     double inv_req2;    // 1/r_eq^2
-    double to_unit[3];  // 2^32 / L: positions as 32-bit fractions of the box
-    float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_unit[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
+    float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
 };
 
 static PC make_pc(const fipi_ctx* ctx) {
@@ -98,8 +97,6 @@ static PC make_pc(const fipi_ctx* ctx) {
         c.mdc[a] = c.margin / c.dc[a];
         c.f_dc[a] = (float)c.dc[a];
         c.img[a] = c.dc[a] * (c.nc[a] - 2);
-        c.to_unit[a] = 4294967296.0 / c.L[a];
-        c.f_unit[a] = (float)(c.L[a] / 4294967296.0);
     }
     c.drag = 6.0 * c.pi * c.mu;
     c.f_req = (float)c.r_eq;
@@ -362,27 +359,21 @@ __global__ void k_cells_place(PC pc, const double* __restrict__ p, const unsigne
     }
 }
 
-// What the contact forces (k_f_pp_warp) read of particle i at sorted position
-// s: its position relative to its cell in FP32 with the id and, with ipos
-// (mixed form, by id), as 32-bit fractions of the box (2^32 wraps to 0, as
-// the box does).
+// What the contact forces read of particle i at sorted position s: its
+// position relative to its cell in FP32, and the id.
 __device__ __forceinline__ void sorted_pos(const PC& pc, const double* __restrict__ p, int i, int cx, int cy, int cz,
-                                           int s, float4* spos, int4* ipos) {
+                                           int s, float4* spos) {
     const int n = pc.n;
     const double x = p[i], y = p[n + i], z = p[2 * n + i];
     spos[s] = make_float4((float)fma((double)-cx, pc.dc[0], x), (float)fma((double)-cy, pc.dc[1], y),
                           (float)fma((double)-cz, pc.dc[2], z), __int_as_float(i));
-    if (ipos)
-        ipos[i] = make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(x * pc.to_unit[0]),
-                            (int)(unsigned)(unsigned long long)__double2ll_rn(y * pc.to_unit[1]),
-                            (int)(unsigned)(unsigned long long)__double2ll_rn(z * pc.to_unit[2]), 0);
 }
 
 // One warp per cell: rank of each id among the cell's ids.  With spos the
 // sorted positions of the contact forces are written as well.
 __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __restrict__ off, int ncells,
                               const unsigned* __restrict__ tmp, unsigned* ids, unsigned* skeys,
-                              unsigned long long* ymax, int* it_mark, float4* spos, int4* ipos) {
+                              unsigned long long* ymax, int* it_mark, float4* spos) {
     const int cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (ymax && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -399,7 +390,7 @@ __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __
         for (int j = beg; j < end; ++j) r += tmp[j] < id;
         ids[beg + r] = id;
         skeys[beg + r] = (unsigned)cell;
-        if (spos) sorted_pos(pc, p, (int)id, cx, cy, cz, beg + r, spos, ipos);
+        if (spos) sorted_pos(pc, p, (int)id, cx, cy, cz, beg + r, spos);
     }
 }
 
@@ -423,7 +414,7 @@ static bool build_cells(fipi_ctx* ctx, const double* p_dev, bool want_it_mark = 
     }
     { LaunchScope ls_(ctx, "cell offsets", 0.0); k_cells_scan<<<1, 1024, 0, ctx->stream>>>(b.cell_cnt, b.ncells, b.cell_off); }
     { LaunchScope ls_(ctx, "cell placement", 0.0); k_cells_place<<<nb, kPT, 0, ctx->stream>>>(pc, p_dev, b.keys_alt, b.ids_alt, b.cell_off, b.keys, ym); }
-    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos, b.ipos); }
+    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos); }
     std::swap(b.keys, b.keys_alt);  // sorted keys now in keys
     return want_it_mark;
 }
@@ -559,12 +550,11 @@ __global__ void k_f_pp(PC pc, const double* __restrict__ p, const unsigned* __re
 
 // k_cells_order's sorted positions, for callers that built the list without them.
 __global__ void k_sorted_pos(PC pc, const double* __restrict__ p, const unsigned* __restrict__ keys,
-                             const unsigned* __restrict__ ids, float4* __restrict__ spos, int4* __restrict__ ipos) {
+                             const unsigned* __restrict__ ids, float4* __restrict__ spos) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= pc.n) return;
     const unsigned key = keys[s];
-    sorted_pos(pc, p, (int)ids[s], key % pc.nc[0], (key / pc.nc[0]) % pc.nc[1], key / (pc.nc[0] * pc.nc[1]), s, spos,
-               ipos);
+    sorted_pos(pc, p, (int)ids[s], key % pc.nc[0], (key / pc.nc[0]) % pc.nc[1], key / (pc.nc[0] * pc.nc[1]), s, spos);
 }
 
 // Mixed-form contact forces when every axis has at least 4 cells.  Then
@@ -729,19 +719,15 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
 // d_cell).  About one candidate in twelve lies within r_eq (4/3 pi r_eq^3
 // against 27 cells), so these separations only select: candidates within
 // r_eq plus their rounding bound (f_req2_sel) are queued by ballot, and every
-// 32 of them are evaluated with all lanes busy.  The evaluation takes the
-// minimum image of cluster.cpp:225-232 (shift d by L when |d| exceeds
-// d_cell (n_cell - 2)):
-//  FP64 form   the rule itself on the FP64 positions (FP64 issues at 1/64 of
-//              the FP32 rate: 40 pairs a particle instead of 500);
-//  mixed form  positions as 32-bit fractions of the box, whose wrapping
-//              difference is the nearest image: exact to L 2^-32 (FP32 cell
-//              coordinates: d_cell 2^-23), then FP32.
-// Both select and evaluate the same image as the rule for every pair that
+// 32 of them are evaluated with all lanes busy, in FP64 from the FP64
+// positions with the minimum-image rule of cluster.cpp:225-232 (shift d by L
+// when |d| exceeds d_cell (n_cell - 2)).  FP64 issues at 1/64 of the FP32 rate:
+// 40 pairs a particle instead of 500.  The selection sees the same image as
+// the rule for every pair that
 // can interact: with at least 4 cells per axis the rule shifts exactly the
 // pairs reached through the periodic wrap, and with 3 it differs only for
 // pairs further apart than d_cell; f_pp_path asks for r_eq <= d_cell
-// there, and for r_eq < L / 2.  Lane sums meet in a fixed shuffle order:
+// there.  Lane sums meet in a fixed shuffle order:
 // deterministic.
 constexpr int kFppWarps = 4;
 constexpr int kFppStage = 768;  // staged candidates (12 KB); more go in several rounds
@@ -902,10 +888,8 @@ __device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict
     }
 }
 
-template <typename TA>
 __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const double* __restrict__ p,
                                                               const float4* __restrict__ spos,
-                                                              const int4* __restrict__ ipos,
                                                               const int* __restrict__ off,
                                                               const double* __restrict__ rmp_p,
                                                               const double* __restrict__ f_pi,
@@ -920,62 +904,33 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const doubl
     fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
         const int i = __float_as_int(h.w);
         const bool tau_on = mark && any_force(f_pi, n, i);
-        TA ax = TA(0), ay = TA(0), az = TA(0), tau = TA(0);
-        if constexpr (sizeof(TA) == sizeof(float)) {
-            const float req = pc.f_req, str = (float)*rmp_p * pc.f_kn;
-            const int4 hi = ipos[i];
-            walk([&](int j) {
-                const int4 c = ipos[j];
-                float dx = (float)(int)((unsigned)hi.x - (unsigned)c.x) * pc.f_unit[0];
-                float dy = (float)(int)((unsigned)hi.y - (unsigned)c.y) * pc.f_unit[1];
-                float dz = (float)(int)((unsigned)hi.z - (unsigned)c.z) * pc.f_unit[2];
-                float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                if (d2 == 0.f) {  // coincident
-                    double d[3];
-                    coincident_d(min(i, j), max(i, j), pc.r_p, d);
-                    const float sg = i < j ? 1.f : -1.f;
-                    dx = sg * (float)d[0];
-                    dy = sg * (float)d[1];
-                    dz = sg * (float)d[2];
-                    d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                }
-                // 1/|d|: the FP32 estimate and one Newton step
-                float y = rsqrtf(d2);
-                y = fmaf(0.5f * y, fmaf(-(d2 * y), y, 1.f), y);
-                const float dn = d2 * y;
-                if (!(dn < req)) return;
-                const float sc = (req - dn) * (str * y);  // the force is sc d
-                ax = fmaf(dx, sc, ax);
-                ay = fmaf(dy, sc, ay);
-                az = fmaf(dz, sc, az);
-                if (tau_on && i < j) tau = fmaf(0.5f * sc, d2, tau);
-            });
-        } else {
-            const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
-            const double str = *rmp_p * pc.k_n;
-            walk([&](int j) {
-                double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
-                               min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
-                double d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
-                if (!nonzero_bits(d2) && !nonzero_bits(d[0]) && !nonzero_bits(d[1]) && !nonzero_bits(d[2])) {
-                    coincident_d(min(i, j), max(i, j), pc.r_p, d);
-                    if (j < i)
-                        for (int a = 0; a < 3; ++a) d[a] = -d[a];
-                    d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
-                }
-                // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
-                const double sc = fma(inv_distance(d2 * pc.inv_req2), str, -str);
-                if (!(sc > 0.0)) return;
-                ax = fma(d[0], sc, ax);
-                ay = fma(d[1], sc, ay);
-                az = fma(d[2], sc, az);
-                if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
-            });
-        }
-        const TA t = warp_total4(ax, ay, az, tau, lane);
+        double ax = 0.0, ay = 0.0, az = 0.0, tau = 0.0;
+        const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
+        const double str = *rmp_p * pc.k_n;
+        walk([&](int j) {
+            double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
+                           min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
+            double d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+            if (!nonzero_bits(d2) && !nonzero_bits(d[0]) && !nonzero_bits(d[1]) && !nonzero_bits(d[2])) {
+                coincident_d(min(i, j), max(i, j), pc.r_p, d);
+                if (j < i)
+                    for (int a = 0; a < 3; ++a) d[a] = -d[a];
+                d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+            }
+            // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
+            const double y = inv_distance(d2 * pc.inv_req2);
+            const long long yb = __double_as_longlong(y);
+            if (yb <= 0x3ff0000000000000ll || yb > 0x7ff0000000000000ll) return;  // !(y > 1), on the bits
+            const double sc = fma(y, str, -str);
+            ax = fma(d[0], sc, ax);
+            ay = fma(d[1], sc, ay);
+            az = fma(d[2], sc, az);
+            if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
+        });
+        const double t = warp_total4(ax, ay, az, tau, lane);
         if (on && (lane & 7) == 0) {
-            if (lane < 24) f_pp[(lane >> 3) * n + i] = (double)t;
-            else if (tau_part) tau_part[i] = (double)t;
+            if (lane < 24) f_pp[(lane >> 3) * n + i] = t;
+            else if (tau_part) tau_part[i] = t;
         }
     });
 }
@@ -1637,21 +1592,20 @@ static void it_mark_launch(fipi_ctx* ctx, const double* p) {
 // accumulated per particle (tau_part) and summed when it is asked for.
 //
 // Mixed form with at least 4 cells per axis: k_f_pp_fast.  The FP64 form, and
-// 3 cells on an axis: k_f_pp_warp wherever its cell offsets give the minimum
-// image (see there); otherwise (margin != 0, 3 cells on an axis and r_eq >
-// d_cell, r_eq >= L/2) k_f_pp, one warp per home cell in the reference's pair
-// order.  Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp
-// 110; 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 12; mixed,
-// 20,000 particles, k_f_pp_fast 27, k_f_pp_warp 32.
+// the mixed form with 3 cells on an axis (where its separations always came
+// from FP64 differences): k_f_pp_warp wherever its cell offsets give the
+// minimum image (see there); otherwise (margin != 0, or 3 cells on an axis and
+// r_eq > d_cell) k_f_pp, one warp per home cell in the reference's pair order.
+// Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp 110;
+// 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 16; mixed, 20,000
+// particles, k_f_pp_fast 27.
 enum class FppPath { cell, warp, fast };
 static FppPath f_pp_path(const fipi_ctx* ctx, bool fp32) {
     const ParticleBufs& b = ctx->pb;
     if (fp32 && b.ncell[0] >= 4 && b.ncell[1] >= 4 && b.ncell[2] >= 4) return FppPath::fast;
-    const double L[3] = {ctx->P.lx, ctx->P.ly, ctx->P.lz};
     if (ctx->P.margin != 0.0) return FppPath::cell;
     for (int a = 0; a < 3; ++a)
-        if (b.ncell[a] < 3 || (b.ncell[a] == 3 && ctx->P.r_eq > b.dcell[a]) || !(ctx->P.r_eq < 0.5 * L[a]))
-            return FppPath::cell;
+        if (b.ncell[a] < 3 || (b.ncell[a] == 3 && ctx->P.r_eq > b.dcell[a])) return FppPath::cell;
     return FppPath::warp;
 }
 
@@ -1663,14 +1617,14 @@ static void f_pp_launch(fipi_ctx* ctx, const double* p, const double* rmp, const
     if (tau && !have_it_mark) it_mark_launch(ctx, p);
     const FppPath path = f_pp_path(ctx, sizeof(TA) == sizeof(float));
     if (path != FppPath::cell) {
-        if (!have_spos) { LaunchScope ls_(ctx, "sorted FP32 positions", 0.0); k_sorted_pos<<<(b.n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, b.keys, b.ids, b.spos, b.ipos); }
+        if (!have_spos) { LaunchScope ls_(ctx, "sorted FP32 positions", 0.0); k_sorted_pos<<<(b.n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, b.keys, b.ids, b.spos); }
         LaunchScope ls_(ctx, "contact forces", 0.0);
         if (path == FppPath::fast)
             k_f_pp_fast<<<b.ncells, 32 * kFppRows, 0, ctx->stream>>>(pc, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr,
                                                                      b.it_mark, f_pp, tau ? b.tau_part : nullptr);
         else
-            k_f_pp_warp<TA><<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
-                pc, p, b.spos, b.ipos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp,
+            k_f_pp_warp<<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
+                pc, p, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp,
                 tau ? b.tau_part : nullptr);
     } else {
         const int blocks = (b.ncells * 32 + 255) / 256;
@@ -1818,8 +1772,6 @@ fipi_status particles_alloc(fipi_ctx* ctx) {
     FIPI_CUDA(ctx, A((void**)&b.hist, sizeof(unsigned) * b.hist_cap));
     FIPI_CUDA(ctx, A((void**)&b.tau_part, sizeof(double) * n));
     FIPI_CUDA(ctx, A((void**)&b.spos, sizeof(float4) * n));
-    // the mixed form's k_f_pp_warp reads box fractions instead of the FP64 positions
-    if (ctx->prec == FIPI_MIXED && f_pp_path(ctx, true) == FppPath::warp) FIPI_CUDA(ctx, A((void**)&b.ipos, sizeof(int4) * n));
     FIPI_CUDA(ctx, A((void**)&b.sp_fw, sizeof(double) * 6 * n));
     FIPI_CUDA(ctx, A((void**)&b.ymax, sizeof(unsigned long long) * 2));
     {
@@ -1837,7 +1789,7 @@ void particles_free(fipi_ctx* ctx) {
     ParticleBufs& b = ctx->pb;
     void* all[] = {b.p, b.p_old, b.u_old, b.f_pp, b.f_pi, b.r, b.cth, b.keys, b.keys_alt, b.ids, b.ids_alt,
                    b.cell_off, b.cell_cnt, b.sp_keys, b.sp_keys_alt, b.sp_vals, b.sp_vals_alt, b.sp_prev,
-                   b.hist, b.tau_part, b.it_mark, b.tau, b.spos, b.ipos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
+                   b.hist, b.tau_part, b.it_mark, b.tau, b.spos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
     for (void* p : all)
         if (p) cudaFree(p);
     b = ParticleBufs{};
