@@ -440,12 +440,59 @@ fipi_status ck_reserve(fipi_ctx* ctx, int slots) {
     return FIPI_OK;
 }
 
+// All regions of a checkpoint in one launch (fourteen copies of their own cost
+// more to start than to run on small grids).  Sizes are multiples of 8 bytes,
+// addresses of 16.
+constexpr int kMaxRegions = 24;
+struct CkList {
+    const uint4* src[kMaxRegions];
+    uint4* dst[kMaxRegions];
+    size_t bytes[kMaxRegions];
+    int n;
+};
+__global__ void __launch_bounds__(256) k_copy_regions(CkList l) {
+    const size_t stride = (size_t)gridDim.x * 256, at = (size_t)blockIdx.x * 256 + threadIdx.x;
+    for (int r = 0; r < l.n; ++r) {
+        const uint4* __restrict__ src = l.src[r];
+        uint4* __restrict__ dst = l.dst[r];
+        const size_t units = l.bytes[r] / 16;
+        size_t i = at;
+        for (; i + 3 * stride < units; i += 4 * stride) {
+            const uint4 v0 = __ldcs(src + i), v1 = __ldcs(src + i + stride), v2 = __ldcs(src + i + 2 * stride),
+                        v3 = __ldcs(src + i + 3 * stride);
+            dst[i] = v0;
+            dst[i + stride] = v1;
+            dst[i + 2 * stride] = v2;
+            dst[i + 3 * stride] = v3;
+        }
+        for (; i < units; i += stride) dst[i] = src[i];
+        if (at == 0 && (l.bytes[r] & 8))
+            reinterpret_cast<unsigned long long*>(dst + units)[0] = reinterpret_cast<const unsigned long long*>(src + units)[0];
+    }
+}
+fipi_status ck_copy(fipi_ctx* ctx, unsigned char* base, bool save) {
+    CkList l{};
+    size_t total = 0;
+    for (const CkCopy& c : ck_regions(ctx, base)) {
+        l.src[l.n] = (const uint4*)(save ? c.ctxbuf : c.slot);
+        l.dst[l.n] = (uint4*)(save ? c.slot : c.ctxbuf);
+        l.bytes[l.n++] = c.bytes;
+        total += c.bytes;
+    }
+    const size_t blocks = std::min<size_t>((size_t)ctx->num_sms * 8, total / (16 * 256) + 1);
+    {
+        LaunchScope ls(ctx, save ? "checkpoint save" : "checkpoint load", 2.0 * (double)total);
+        k_copy_regions<<<(unsigned)blocks, 256, 0, ctx->stream>>>(l);
+    }
+    FIPI_CUDA(ctx, cudaGetLastError());
+    return FIPI_OK;
+}
+
 fipi_status ck_save(fipi_ctx* ctx, int slot) {
     fipi_status st = slot_ok(ctx, slot);
     if (st != FIPI_OK) return st;
-    unsigned char* base = ctx->ck.base + (size_t)slot * ctx->ck.bytes;
-    for (const CkCopy& c : ck_regions(ctx, base))
-        FIPI_CUDA(ctx, cudaMemcpyAsync(c.slot, c.ctxbuf, c.bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    st = ck_copy(ctx, ctx->ck.base + (size_t)slot * ctx->ck.bytes, true);
+    if (st != FIPI_OK) return st;
     ctx->ck.t[slot] = ctx->t;
     return FIPI_OK;
 }
@@ -454,9 +501,8 @@ fipi_status ck_load(fipi_ctx* ctx, int slot) {
     fipi_status st = slot_ok(ctx, slot);
     if (st != FIPI_OK) return st;
     if (ctx->ck.t[slot] < 0) return set_error(ctx, FIPI_ERR_STATE, "checkpoint slot is empty");
-    unsigned char* base = ctx->ck.base + (size_t)slot * ctx->ck.bytes;
-    for (const CkCopy& c : ck_regions(ctx, base))
-        FIPI_CUDA(ctx, cudaMemcpyAsync(c.ctxbuf, c.slot, c.bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    st = ck_copy(ctx, ctx->ck.base + (size_t)slot * ctx->ck.bytes, false);
+    if (st != FIPI_OK) return st;
     ctx->t = ctx->ck.t[slot];
     set_tick(ctx, ctx->t);
     ctx->pb.tau_valid = false;
@@ -494,9 +540,9 @@ void adjoint_fields(fipi_ctx* ctx, bool first) {
     const fipi_params& P = ctx->P;
     OpAdjStokes<D> os{{S[0], S[1], S[2], S[3], S[4]},
                       {a.lamF, a.lamF + V, a.lamF + 2 * V},
-                      {(const D*)ctx->fb.g[0], (const D*)ctx->fb.g[1], (const D*)ctx->fb.g[2]},
-                      a.tmu,
-                      (const D*)ctx->fb.c,
+                      {a.in.g1[0], a.in.g1[1], a.in.g1[2]},
+                      a.in.mu,
+                      a.in.c1,
                       particles_on(ctx) ? a.part : nullptr,
                       V,
                       k.lam_eps,
@@ -511,11 +557,10 @@ void adjoint_fields(fipi_ctx* ctx, bool first) {
                   first ? 1 : 0, ctx->conserve_mass};
     launch_z<D, 5, -1>(ctx, "adjoint: Z forward + CH", 13, zc);
     {
-        // mobility and lambda through the CH update (c_hat^{n+1} = chat, f^n = fhat_old after the
-        // recomputed step, f^{n-1} taped before it)
+        // mobility and lambda through the CH update (c_hat^{n+1}, f^n and f^{n-1})
         LaunchScope ls(ctx, "adjoint: CH parameter sums", 4.0 * g.SH * sizeof(CD));
-        k_adj_param_ch<<<kParamBlocks, 256, 0, ctx->stream>>>(S[2], sp(ctx->fb.chat), sp(ctx->fb.fhat_old),
-                                                               sp(a.tfo), kt, k, P.mobility, first ? 1 : 0, g.ny,
+        k_adj_param_ch<<<kParamBlocks, 256, 0, ctx->stream>>>(S[2], (const CD*)a.in.chat1, (const CD*)a.in.fhat0,
+                                                               (const CD*)a.in.fo, kt, k, P.mobility, first ? 1 : 0, g.ny,
                                                                g.h, (size_t)g.SH, a.pg_part);
     }
     const double invV = 1.0 / (double)g.V;
@@ -527,9 +572,9 @@ void adjoint_fields(fipi_ctx* ctx, bool first) {
     launch_z<D, 2, +1>(ctx, "adjoint: Z inverse", 4, zi2);
     launch_y<D>(ctx, 2, Sv, Sv, +1);
     OpAdjCH<D> oc{{S[0], S[1], S[2], S[3]},
-                  a.tc0,
-                  {a.tg0, a.tg0 + V, a.tg0 + 2 * V},
-                  {a.tu, a.tu + V, a.tu + 2 * V},
+                  a.in.c0,
+                  {a.in.g0, a.in.g0 + V, a.in.g0 + 2 * V},
+                  {a.in.u, a.in.u + V, a.in.u + 2 * V},
                   {a.la_u, a.la_u + V, a.la_u + 2 * V},
                   k.lam_eps,
                   g.nx,
@@ -575,6 +620,9 @@ fipi_status adjoint_step_impl(fipi_ctx* ctx, int slot) {
     enqueue_step(ctx);
     ctx->tape_u[0] = ctx->tape_u[1] = ctx->tape_u[2] = nullptr;
     ctx->tape_mu = nullptr;
+    a.in = AdjBufs::In{a.tc0, a.tg0, a.tu, a.tmu, a.tp0, a.tfpp0, a.tfo, (const D*)b.c,
+                       {(const D*)b.g[0], (const D*)b.g[1], (const D*)b.g[2]}, b.chat, b.fhat_old, ctx->pb.r,
+                       ctx->pb.cth};
     if (parts) {
         st = particles_adjoint(ctx);
         if (st != FIPI_OK) return st;
@@ -600,24 +648,15 @@ fipi_status adjoint_reverse_pair(fipi_ctx* ctx, int slot_n, int slot_n1, const d
     const CkLayout L = ck_layout(ctx);
     const unsigned char* sn = ctx->ck.base + (size_t)slot_n * ctx->ck.bytes;
     const bool parts = particles_on(ctx);
-    // inputs of the reverse pass from the step's start state
-    FIPI_CUDA(ctx, cudaMemcpyAsync(a.tc0, sn + L.c, sizeof(D) * V, cudaMemcpyDeviceToDevice, ctx->stream));
-    FIPI_CUDA(ctx, cudaMemcpyAsync(a.tg0, sn + L.g, sizeof(D) * 3 * V, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (n > 0)  // f_hat^{n-1}: the start state's f_hat history (spectral region 3 of the slot)
-        FIPI_CUDA(ctx, cudaMemcpyAsync(a.tfo, sn + L.spec + 3 * 2 * sizeof(D) * SH, sizeof(CD) * SH,
-                                       cudaMemcpyDeviceToDevice, ctx->stream));
-    if (parts) {
-        const size_t b3 = sizeof(D) * 3 * (size_t)ctx->pb.n;
-        FIPI_CUDA(ctx, cudaMemcpyAsync(a.tp0, sn + L.p, b3, cudaMemcpyDeviceToDevice, ctx->stream));
-        FIPI_CUDA(ctx, cudaMemcpyAsync(a.tfpp0, sn + L.fpp, b3, cudaMemcpyDeviceToDevice, ctx->stream));
-        set_tick(ctx, n);  // ramp(n + 1, 0.2 t_end) of the reversed step
-        FIPI_CUDA(ctx, cudaMemcpyAsync(a.rmp, ctx->d_rmp, sizeof(D), cudaMemcpyDeviceToDevice, ctx->stream));
-    }
-    FIPI_CUDA(ctx, cudaMemcpyAsync(a.tu, tape, sizeof(D) * 3 * V, cudaMemcpyDeviceToDevice, ctx->stream));
-    FIPI_CUDA(ctx, cudaMemcpyAsync(a.tmu, tape + 3 * V, sizeof(D) * V, cudaMemcpyDeviceToDevice, ctx->stream));
-    // the step's end state, as the recomputed step would have left it
-    fipi_status st = ck_load(ctx, slot_n1);
-    if (st != FIPI_OK) return st;
+    // the reverse pass reads the states before and after the step where they are
+    const unsigned char* s1 = ctx->ck.base + (size_t)slot_n1 * ctx->ck.bytes;
+    auto spec = [&](const unsigned char* slot, int i) { return slot + L.spec + (size_t)i * sizeof(CD) * SH; };
+    const D* g1 = (const D*)(s1 + L.g);
+    a.in = AdjBufs::In{(const D*)(sn + L.c), (const D*)(sn + L.g), tape, tape + 3 * V, (const D*)(sn + L.p),
+                       (const D*)(sn + L.fpp), spec(sn, 3), (const D*)(s1 + L.c), {g1, g1 + V, g1 + 2 * V},
+                       spec(s1, 0), spec(s1, 3), (const D*)(s1 + L.r), (const D*)(s1 + L.cth)};
+    if (parts) set_ramp(ctx, n, a.rmp);  // ramp(n + 1, 0.2 t_end) of the reversed step
+    fipi_status st = FIPI_OK;
     if (parts) {
         st = particles_adjoint(ctx);
         if (st != FIPI_OK) return st;
@@ -944,6 +983,9 @@ fipi_status fipi_trajectory_backward(fipi_ctx* ctx, const double* dc, const doub
         st = check_status(ctx);
         if (st != FIPI_OK) return st;
     }
+    // the context is left in the state after the trajectory's first step
+    st = ck_load(ctx, tr->K + 1);
+    if (st != FIPI_OK) return st;
     tr->t0 = -1;  // the state is no longer the trajectory's end
     return FIPI_OK;
 }

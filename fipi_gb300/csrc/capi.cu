@@ -273,7 +273,6 @@ extern "C" {
 static fipi_status set_phase_impl(fipi_ctx* ctx, const double* c, bool dev) {
     if (!ctx || !c) return set_error(ctx, FIPI_ERR_BAD_ARG, "NULL argument");
     FIPI_CUDA(ctx, cudaSetDevice(ctx->device));
-    graphs_reset(ctx);
     fipi_status st = fields_set_phase(ctx, c, dev);
     if (st != FIPI_OK) return st;
     ctx->t = 0;

@@ -59,20 +59,15 @@ struct ParticleBufs {
     unsigned* ids_alt = nullptr;   // n
     int* cell_off = nullptr;       // ncells + 1
     int* cell_cnt = nullptr;       // ncells
-    // spreading records (8 per particle)
-    unsigned* sp_keys = nullptr;      // 8n node index
-    unsigned* sp_keys_alt = nullptr;  // 8n
-    unsigned* sp_vals = nullptr;      // 8n record id = particle*8 + corner
-    unsigned* sp_vals_alt = nullptr;  // 8n
+    // spreading: node lists of the FP64 form (particles.cu, NodeLists)
+    int* sp_head = nullptr;           // V, -1 between spreads
+    int* sp_next = nullptr;           // 8n
     unsigned* sp_prev = nullptr;      // 8n nodes written by the previous spread
     // mixed form: per node 32 bytes, the three fixed-point spread sums and,
     // in the low half of the fourth word, the FP32 sum of |contribution|
     // (the range bound): one 32-byte sector per touched node
     unsigned long long* sp_acc = nullptr;
     int sp_prev_valid = 0;
-    // radix sort scratch
-    unsigned* hist = nullptr;  // 256 * max_blocks
-    int hist_cap = 0;
     // diagnostics
     double* tau_part = nullptr;  // n, per-particle packing-energy terms
     float4* spos = nullptr;      // n, sorted cell-relative FP32 positions + id
@@ -133,10 +128,9 @@ struct AdjBufs {
     double* lamF2 = nullptr;   // cotangent of the stage-2 contact forces
     double* lam_p1 = nullptr;  // cotangent of p1
     double* lamloc = nullptr;  // 8n cotangents of `loc`
-    unsigned* rk = nullptr;    // 16n spreading records (node, record) + ping-pong
-    unsigned* rv = nullptr;
-    unsigned* rk2 = nullptr;
-    unsigned* rv2 = nullptr;
+    unsigned* rnode = nullptr;  // 16n interpolation records: node and list link
+    int* rnext = nullptr;
+    bool part_valid = false;    // `part` is zero except at the nodes in rnode
     double* rw = nullptr;      // 14n: fractions (3) and cotangents (4) of 2n interpolations
     double* rmp = nullptr;     // 1: ramp factor of the reversed step
     // parameter cotangents, summed from fipi_adjoint_seed over every reversed step
@@ -147,6 +141,15 @@ struct AdjBufs {
     double* dct = nullptr;      // n: cotangent of each particle's cos(theta)
     double* pp_sig = nullptr;   // n: per-particle terms of the sigma (f_pi) cotangent of one step
     double* pp_kn = nullptr;    // n: per-particle terms of the k_n cotangent of one step
+    // what a reversed step reads: the states before (0) and after (1) the step
+    // and its tape, in the buffers above or in checkpoint slots
+    struct In {
+        const double *c0 = nullptr, *g0 = nullptr, *u = nullptr, *mu = nullptr, *p0 = nullptr, *fpp0 = nullptr;
+        const void* fo = nullptr;  // f_hat^{n-1}
+        const double *c1 = nullptr, *g1[3] = {};
+        const void *chat1 = nullptr, *fhat0 = nullptr;  // c_hat^{n+1}, f_hat^n
+        const double *r = nullptr, *cth = nullptr;
+    } in;
     // per-step tapes of a trajectory segment (u^n, mu^{n+1}: 4V doubles each)
     double* seg_tape = nullptr;
     int seg_tape_steps = 0;
@@ -293,6 +296,8 @@ fipi_status particles_wrap(fipi_ctx* ctx, double* p_host);
 void enqueue_step(fipi_ctx* ctx);  // one forward step, direct launches
 // Sets the device step index and the ramp factor of step t (particles.cu).
 void set_tick(fipi_ctx* ctx, int t);
+// *rmp = ramp(t + 1, 0.2 t_end).
+void set_ramp(fipi_ctx* ctx, int t, double* rmp);
 // Particle stages of the step reversed (after the taped forward step):
 // la_p, la_fpp of the end state -> la_p of the start state (stage part) and
 // the particle cotangents `part` on c^{n+1}, grad c^{n+1}.

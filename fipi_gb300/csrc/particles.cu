@@ -2,9 +2,9 @@
 // cluster.cpp / element.cpp of the reference).
 //
 //  - cell list: key = i + j n + k n^2 with i = floor(p/d_cell + margin/d_cell)
-//    (cluster.cpp:140-165), a stable LSD radix sort of (key, particle id) and
-//    offsets by binary search; ids inside a cell are ascending, which is the
-//    order the reference's linked lists hold them in (linked_list.cpp:30-43);
+//    (cluster.cpp:140-165), counts, offsets and ranks; ids inside a cell are
+//    ascending, which is the order the reference's linked lists hold them in
+//    (linked_list.cpp:30-43);
 //  - contact forces (cluster.cpp:174-275) gathered per particle over the 27
 //    neighbour cells with the reference's sign rule, summed in a fixed
 //    order: deterministic and atomic-free (k_f_pp_warp, k_f_pp_fast; k_f_pp,
@@ -12,10 +12,9 @@
 //    they do not take and for the pair lists);
 //  - interpolation, attachment force, Heun advection and periodic wrap per
 //    particle (field.cpp:223-248, element.cpp:55-185);
-//  - spreading (cluster.cpp:344-410) as a sorted segmented reduction: the
-//    8 corner records of every particle are radix-sorted by grid node,
-//    stable in particle id, and each node sums its records in ascending id,
-//    the order in which the reference's loop adds them.
+//  - spreading (cluster.cpp:344-410): the 8 corner records of every particle
+//    are listed by grid node and each node sums its records in ascending
+//    particle id, the order in which the reference's loop adds them.
 //
 // Positions are FP64 in every form.  This file is compiled with
 // -fmad=false so its FP64 expressions round exactly as the reference's.
@@ -211,19 +210,6 @@ __global__ void k_rs_scatter(const unsigned* __restrict__ kin, const unsigned* _
     }
 }
 
-// Sorts (k, v) by the low `bits` bits of k; results end in (k, v).
-static void radix_sort(fipi_ctx* ctx, unsigned*& k, unsigned*& v, unsigned*& k2, unsigned*& v2, int n, int bits) {
-    if (n <= 0) return;
-    const int nblk = (n + RS_TILE - 1) / RS_TILE;
-    for (int shift = 0; shift < bits; shift += 8) {
-        { LaunchScope ls_(ctx, "radix sort hist", 0.0); k_rs_hist<<<nblk, RS_T, 0, ctx->stream>>>(k, n, shift, ctx->pb.hist, nblk); }
-        { LaunchScope ls_(ctx, "radix sort scan", 0.0); k_scan_excl<<<1, 1024, 0, ctx->stream>>>(ctx->pb.hist, 256 * nblk); }
-        { LaunchScope ls_(ctx, "radix sort scatter", 0.0); k_rs_scatter<<<nblk, RS_T, 0, ctx->stream>>>(k, v, k2, v2, n, shift, ctx->pb.hist, nblk); }
-        std::swap(k, k2);
-        std::swap(v, v2);
-    }
-}
-
 static int bits_for(long long maxval) {
     int b = 1;
     while ((1ll << b) <= maxval) ++b;
@@ -233,6 +219,15 @@ static int bits_for(long long maxval) {
 // ------------------------------------------------------------ cell list
 __device__ __forceinline__ int cell_coord(double x, double dcell, double margin) {
     return (int)floor(x / dcell + margin / dcell);  // cluster.cpp:140-142
+}
+
+// The same value by one product, margin/d_cell formed on the host: where the
+// quotient is not within 1e-9 of a cell face its rounding cannot change the
+// floor (|quotient| < 1e5: errors below 4e-11); otherwise the division.
+__device__ __forceinline__ int cell_coord_fast(double x, double dcell, double margin, double inv_dc, double mdc) {
+    const double q = x * inv_dc + mdc, fl = floor(q), fr = q - fl;
+    if (fr > 1e-9 && fr < 1.0 - 1e-9 && fabs(q) < 1e5) return (int)fl;
+    return cell_coord(x, dcell, margin);
 }
 
 // x != 0.0 on the bits (true for NaN, false for -0.0), integer operations only
@@ -256,7 +251,8 @@ __device__ __forceinline__ unsigned cell_key(const PC& pc, double x, double y, d
     const double xs[3] = {x, y, z};
     int c[3];
     for (int a = 0; a < 3; ++a)
-        c[a] = FAST ? (int)floor(fma(xs[a], pc.inv_dc[a], pc.mdc[a])) : cell_coord(xs[a], pc.dc[a], pc.margin);
+        c[a] = FAST ? (int)floor(fma(xs[a], pc.inv_dc[a], pc.mdc[a]))
+                    : cell_coord_fast(xs[a], pc.dc[a], pc.margin, pc.inv_dc[a], pc.mdc[a]);
     const bool fin = finite_bits(x) && finite_bits(y) && finite_bits(z);
     bool bad = !fin;
     for (int a = 0; a < 3; ++a) {
@@ -321,8 +317,9 @@ __global__ void k_cells_count(PC pc, const double* __restrict__ p, unsigned* key
     }
 }
 
-// Exclusive scan of ncells counts into off[0..ncells] (one block).
-__global__ void k_cells_scan(const int* __restrict__ cnt, int ncells, int* off) {
+// Exclusive scan of ncells counts into off[0..ncells] (one block); the counts
+// are zero again afterwards, ready for the next list.
+__global__ void k_cells_scan(int* __restrict__ cnt, int ncells, int* off) {
     __shared__ int part[1024];
     const int t = threadIdx.x;
     const int chunk = (ncells + 1023) / 1024;
@@ -341,6 +338,7 @@ __global__ void k_cells_scan(const int* __restrict__ cnt, int ncells, int* off) 
     for (int i = b; i < e; ++i) {
         off[i] = run;
         run += cnt[i];
+        cnt[i] = 0;
     }
     if (t == 1023) off[ncells] = part[1023];
 }
@@ -394,6 +392,91 @@ __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __
     }
 }
 
+// The whole list in one block for few particles and cells (one launch instead
+// of four, none of which has work for more than a few SMs there): counts,
+// offsets, arrival order and ranks in shared memory, the same results.
+constexpr int kSmallCellsN = 1024, kSmallCells = 4096;
+template <bool FAST>
+__global__ void __launch_bounds__(1024) k_cells_small(PC pc, const double* __restrict__ p, int ncells, int* off,
+                                                      unsigned* ids, unsigned* skeys, int* it_mark, float4* spos,
+                                                      int* status) {
+    __shared__ int start[kSmallCells + 1];  // counts, then offsets
+    __shared__ int part[32];
+    __shared__ unsigned placed[kSmallCellsN], pkey[kSmallCellsN];
+    __shared__ unsigned long long ymax;
+    __shared__ int yfirst;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int n = pc.n;
+    for (int c = t; c <= ncells; c += 1024) start[c] = 0;
+    if (t == 0) {
+        ymax = 0ull;
+        yfirst = 0x7fffffff;
+    }
+    __syncthreads();
+    unsigned key = 0;
+    int slot = 0;
+    unsigned long long yb = 0;
+    if (t < n) {
+        const double y = p[n + t];
+        key = cell_key<FAST>(pc, p[t], y, p[2 * n + t], status);
+        slot = atomicAdd(&start[key], 1);
+        const long long b = __double_as_longlong(y);  // y > 0.0 on the bits (k_cells_count)
+        yb = (b > 0 && b <= 0x7ff0000000000000ll) ? (unsigned long long)b : 0ull;
+        if (it_mark && yb) atomicMax(&ymax, yb);
+    }
+    __syncthreads();
+    if (it_mark && yb && yb == ymax) atomicMin(&yfirst, t);
+    // exclusive scan, a run of consecutive cells per thread
+    const int chunk = (ncells + 1023) / 1024, b = t * chunk, e = min(ncells, b + chunk);
+    int sum = 0;
+    for (int c = b; c < e; ++c) sum += start[c];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) part[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        int v = part[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        part[lane] = v;
+    }
+    __syncthreads();
+    int run = incl - sum + (w > 0 ? part[w - 1] : 0);
+    for (int c = b; c < e; ++c) {
+        const int cnt = start[c];
+        start[c] = run;
+        off[c] = run;
+        run += cnt;
+    }
+    if (t == 0) {
+        start[ncells] = n;
+        off[ncells] = n;
+        if (it_mark && ymax != 0ull) *it_mark = yfirst;
+    }
+    __syncthreads();
+    if (t < n) {
+        placed[start[key] + slot] = (unsigned)t;
+        pkey[start[key] + slot] = key;
+    }
+    __syncthreads();
+    if (t < n) {
+        const unsigned id = placed[t], k = pkey[t];
+        const int beg = start[k], end = start[k + 1];
+        int r = beg;
+        for (int j = beg; j < end; ++j) r += placed[j] < id;
+        ids[r] = id;
+        skeys[r] = k;
+        if (spos) sorted_pos(pc, p, (int)id, k % pc.nc[0], (k / pc.nc[0]) % pc.nc[1], k / (pc.nc[0] * pc.nc[1]), r, spos);
+    }
+}
+
 // Returns true when it also computed it_mark (asked for by `want_it_mark`).
 // With spos the sorted FP32 positions of the contact forces too;
 // `fast` takes the mixed form's cell keys (cell_key<true>).
@@ -405,8 +488,14 @@ static bool build_cells(fipi_ctx* ctx, const double* p_dev, bool want_it_mark = 
     if (n <= 0) return false;
     const int nb = (n + kPT - 1) / kPT;
     unsigned long long* ym = want_it_mark ? b.ymax : nullptr;
+    if (n <= kSmallCellsN && b.ncells <= kSmallCells) {
+        LaunchScope ls_(ctx, "cell list", 0.0);
+        auto kern = fast ? k_cells_small<true> : k_cells_small<false>;
+        kern<<<1, 1024, 0, ctx->stream>>>(pc, p_dev, b.ncells, b.cell_off, b.ids, b.keys, want_it_mark ? b.it_mark : nullptr,
+                                          spos, ctx->status);
+        return want_it_mark;
+    }
     // keys_alt holds the per-particle keys (by id), ids_alt the arrival slots, then the placed ids
-    cudaMemsetAsync(b.cell_cnt, 0, sizeof(int) * (b.ncells + 1), ctx->stream);
     {
         LaunchScope ls_(ctx, "cell keys + counts", 0.0);
         auto kern = fast ? k_cells_count<true> : k_cells_count<false>;
@@ -1365,15 +1454,107 @@ __device__ __forceinline__ void cell_and_frac(const PC& pc, double X, double Y, 
     fr[2] = Z / pc.dz - fz;
 }
 
-// Per particle: the 8 corner records (node, particle*8 + corner), the force
-// density f = (f_pp + f_ext)/dx/dy/dz and the fractions (o, p, q) of
-// cluster.cpp:358-366, computed once here instead of once per record.
-template <typename TA>
-__global__ void k_spread_records(PC pc, const double* __restrict__ p, const double* __restrict__ f_pp,
-                                 unsigned* keys, unsigned* vals, TA* __restrict__ fw) {
+// Spreading in ascending particle id without a sort.  Every record (particle
+// * 8 + corner) is pushed onto a linked list of its node (head, next; an
+// arbitrary order); then the record at the head of a list owns the node:
+// it brings the list into ascending order, sums it in that order (the order of
+// the reference's loop, cluster.cpp:368-406, so the sums are the same
+// whatever the order of the pushes) and leaves the head empty (-1) for the next
+// spread.  Two launches for what took a radix sort of the records in twelve:
+// FP64, 256 particles at 64^3 102 -> 25 us, 20,000 at 256^3 173 -> 63 (sums of
+// launches timed one by one).
+//
+// Records 8n of a push: node, and the list links.
+struct NodeLists {
+    int* head;        // per grid node, -1 = empty
+    int* next;        // per record
+    unsigned* nodes;  // per record
+};
+__device__ __forceinline__ void push_record(const NodeLists& nl, int rec, unsigned node) {
+    nl.nodes[rec] = node;
+    nl.next[rec] = atomicExch(&nl.head[node], rec);
+}
+// Ascending order of the list from `h` (bottom-up merge sort on the links);
+// returns the new first record.
+__device__ __noinline__ int sort_links(int* next, int h) {
+    for (int width = 1;; width *= 2) {
+        int left = h, tail = -1, merges = 0;
+        h = -1;
+        while (left >= 0) {
+            ++merges;
+            int right = left, nl = 0, nr = width;
+            while (nl < width && right >= 0) {
+                right = next[right];
+                ++nl;
+            }
+            while (nl > 0 || (nr > 0 && right >= 0)) {
+                int q;
+                if (nl > 0 && (nr == 0 || right < 0 || left < right)) {
+                    q = left;
+                    left = next[left];
+                    --nl;
+                } else {
+                    q = right;
+                    right = next[right];
+                    --nr;
+                }
+                if (tail < 0) h = q;
+                else next[tail] = q;
+                tail = q;
+            }
+            left = right;
+        }
+        if (tail >= 0) next[tail] = -1;
+        if (merges <= 1) return h;
+    }
+}
+// Calls add(record) for the records of the list owned by `rec` (which is at
+// its head) in ascending order and empties the list.
+template <class Add> __device__ __forceinline__ void owned_records(const NodeLists& nl, int rec, unsigned node, Add&& add) {
+    constexpr int kFew = 8;
+    int few[kFew], m = 0;
+    for (int q = rec; q >= 0; q = nl.next[q]) {
+        if (m < kFew) {
+            int at = m;  // insertion into the ascending prefix
+#pragma unroll
+            for (int k = kFew - 1; k > 0; --k)
+                if (k <= at && few[k - 1] > q) {
+                    few[k] = few[k - 1];
+                    at = k - 1;
+                }
+#pragma unroll
+            for (int k = 0; k < kFew; ++k)
+                if (k == at) few[k] = q;
+        }
+        ++m;
+    }
+    if (m <= kFew) {
+#pragma unroll
+        for (int k = 0; k < kFew; ++k)
+            if (k < m) add(few[k]);
+    } else {
+        for (int q = sort_links(nl.next, rec); q >= 0; q = nl.next[q]) add(q);
+    }
+    nl.head[node] = -1;
+}
+
+// Per particle: its 8 corner records, the force density f = (f_pp + f_ext)/dx
+// /dy/dz and the fractions (o, p, q) of cluster.cpp:358-366, computed once here
+// instead of once per record; with clear_prev the grids are zeroed at the
+// particle's 8 nodes of the previous spread first.
+template <typename TF, typename TA>
+__global__ void k_spread_push(PC pc, const double* __restrict__ p, const double* __restrict__ f_pp, NodeLists nl,
+                              TA* __restrict__ fw, int clear_prev, TF* f0, TF* f1, TF* f2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = pc.n;
     if (i >= n) return;
+    if (clear_prev)
+        for (int c = 0; c < 8; ++c) {
+            const unsigned nd = nl.nodes[8 * i + c];
+            f0[nd] = TF(0);
+            f1[nd] = TF(0);
+            f2[nd] = TF(0);
+        }
     int ix[3];
     double fr[3];
     cell_and_frac(pc, p[i], p[n + i], p[2 * n + i], ix, fr);
@@ -1381,23 +1562,12 @@ __global__ void k_spread_records(PC pc, const double* __restrict__ p, const doub
         const int x = (ix[0] + c_corner[c][0]) % pc.N[0];
         const int y = (ix[1] + c_corner[c][1]) % pc.N[1];
         const int z = (ix[2] + c_corner[c][2]) % pc.N[2];
-        keys[8 * i + c] = (unsigned)(x + (size_t)y * pc.N[0] + (size_t)z * pc.N[0] * pc.N[1]);
-        vals[8 * i + c] = (unsigned)(8 * i + c);
+        push_record(nl, 8 * i + c, (unsigned)(x + (size_t)y * pc.N[0] + (size_t)z * pc.N[0] * pc.N[1]));
     }
     for (int a = 0; a < 3; ++a) {
         fw[a * n + i] = (TA)((f_pp[a * n + i] + 0.0) / pc.dx / pc.dy / pc.dz);
         fw[(3 + a) * n + i] = (TA)fr[a];
     }
-}
-
-template <typename TF>
-__global__ void k_spread_clear(const unsigned* __restrict__ nodes, int m, TF* f0, TF* f1, TF* f2) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= m) return;
-    const unsigned nd = nodes[s];
-    f0[nd] = TF(0);
-    f1[nd] = TF(0);
-    f2[nd] = TF(0);
 }
 
 // Weight products of cluster.cpp:369-406 for corner c, left to right from f.
@@ -1416,58 +1586,43 @@ __device__ __forceinline__ TA corner_value(TA f, int c, TA o, TA pp, TA q) {
 }
 
 template <typename TF, typename TA>
-__global__ void k_spread_reduce(PC pc, const unsigned* __restrict__ keys, const unsigned* __restrict__ vals, int m,
-                                const TA* __restrict__ fw, TF* f0, TF* f1, TF* f2) {
+__global__ void k_spread_sum(int n, NodeLists nl, const TA* __restrict__ fw, TF* f0, TF* f1, TF* f2) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= m) return;
-    const unsigned node = keys[s];
-    if (s > 0 && keys[s - 1] == node) return;
-    const int n = pc.n;
+    if (s >= 8 * n) return;
+    const unsigned node = nl.nodes[s];
+    if (nl.head[node] != s) return;
     TA acc[3] = {TA(0), TA(0), TA(0)};
-    for (int q = s; q < m && keys[q] == node; ++q) {
-        const unsigned rec = vals[q];
-        const int i = (int)(rec >> 3), c = (int)(rec & 7u);
+    owned_records(nl, s, node, [&](int rec) {
+        const int i = rec >> 3, c = rec & 7;
         const TA o = fw[3 * n + i], pp = fw[4 * n + i], qq = fw[5 * n + i];
 #pragma unroll
         for (int a = 0; a < 3; ++a) acc[a] += corner_value<TA>(fw[a * n + i], c, o, pp, qq);
-    }
+    });
     f0[node] = (TF)acc[0];
     f1[node] = (TF)acc[1];
     f2[node] = (TF)acc[2];
 }
 
 // ------------------------------------------------------------ orchestration
-// `step_grid`: the target is the step's persistent spread grid, which only
-// the nodes written by the previous spread need clearing in (the whole grid
-// after a fine-grained call reused the record buffers).
+// clear_prev: f3 is the step's persistent spread grid and nl.nodes the nodes
+// of the previous spread, which are all that needs clearing.
 template <typename T>
-static void spread_t(fipi_ctx* ctx, const double* p, const double* f_pp, T* const f3[3], bool step_grid) {
+static void spread_t(fipi_ctx* ctx, const double* p, const double* f_pp, T* const f3[3], const NodeLists& nl,
+                     bool clear_prev) {
     ParticleBufs& b = ctx->pb;
     const PC pc = make_pc(ctx);
-    const int n = b.n, m = 8 * n;
-    if (step_grid) {
-        if (b.sp_prev_valid) {
-            { LaunchScope ls_(ctx, "spread clear", 0.0); k_spread_clear<T><<<(m + 255) / 256, 256, 0, ctx->stream>>>(b.sp_prev, m, f3[0], f3[1], f3[2]); }
-        } else {
-            for (int a = 0; a < 3; ++a) cudaMemsetAsync(f3[a], 0, sizeof(T) * (size_t)ctx->g.V, ctx->stream);
-        }
-    }
-    { LaunchScope ls_(ctx, "spread records", 0.0); k_spread_records<T><<<(n + 255) / 256, 256, 0, ctx->stream>>>(pc, p, f_pp, b.sp_keys, b.sp_vals, (T*)b.sp_fw); }
-    radix_sort(ctx, b.sp_keys, b.sp_vals, b.sp_keys_alt, b.sp_vals_alt, m, bits_for(ctx->g.V - 1));
-    { LaunchScope ls_(ctx, "spread segmented reduce", 0.0); k_spread_reduce<T, T><<<(m + 255) / 256, 256, 0, ctx->stream>>>(pc, b.sp_keys, b.sp_vals, m, (const T*)b.sp_fw, f3[0], f3[1], f3[2]); }
-    if (step_grid) {
-        cudaMemcpyAsync(b.sp_prev, b.sp_keys, sizeof(unsigned) * m, cudaMemcpyDeviceToDevice, ctx->stream);
-        b.sp_prev_valid = 1;
-    }
+    const int n = b.n;
+    { LaunchScope ls_(ctx, "spread records", 0.0); k_spread_push<T, T><<<(n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, f_pp, nl, (T*)b.sp_fw, clear_prev ? 1 : 0, f3[0], f3[1], f3[2]); }
+    { LaunchScope ls_(ctx, "spread sums", 0.0); k_spread_sum<T, T><<<(8 * n + 127) / 128, 128, 0, ctx->stream>>>(n, nl, (const T*)b.sp_fw, f3[0], f3[1], f3[2]); }
 }
 
 // Mixed-form spreading of the step: the 8 FP32 corner contributions of each
 // particle (the weight products of cluster.cpp:369-406) are added as 64-bit
 // fixed-point integers (units of 2^-32) with atomics.  Integer addition is
 // associative, so the sums do not depend on the order of the atomics (the
-// result is deterministic) and no sort is needed; the touched nodes are
-// then converted to FP32.  The FP64 form keeps the sorted reduction in
-// ascending particle id, bit-identical to the reference.
+// result is deterministic) and no order is needed; the touched nodes are
+// then converted to FP32.  The FP64 form sums in ascending particle id,
+// bit-identical to the reference.
 //
 // Between steps the accumulators are zero everywhere and the force grids are
 // zero except at the 8n nodes of the previous spread (nodes[]): the atomics
@@ -1574,8 +1729,12 @@ void particles_spread(fipi_ctx* ctx) {
     if (ctx->prec == FIPI_MIXED) {
         spread_fx(ctx);
     } else {
+        ParticleBufs& b = ctx->pb;
         double* f3[3] = {(double*)ctx->fb.fsp[0], (double*)ctx->fb.fsp[1], (double*)ctx->fb.fsp[2]};
-        spread_t<double>(ctx, ctx->pb.p, ctx->pb.f_pp, f3, true);
+        if (!b.sp_prev_valid)
+            for (int a = 0; a < 3; ++a) cudaMemsetAsync(f3[a], 0, sizeof(double) * (size_t)ctx->g.V, ctx->stream);
+        spread_t<double>(ctx, b.p, b.f_pp, f3, NodeLists{b.sp_head, b.sp_next, b.sp_prev}, b.sp_prev_valid != 0);
+        b.sp_prev_valid = 1;
     }
 }
 
@@ -1760,16 +1919,16 @@ fipi_status particles_alloc(fipi_ctx* ctx) {
     FIPI_CUDA(ctx, A((void**)&b.ids_alt, sizeof(unsigned) * n));
     FIPI_CUDA(ctx, A((void**)&b.cell_off, sizeof(int) * (b.ncells + 1)));
     FIPI_CUDA(ctx, A((void**)&b.cell_cnt, sizeof(int) * (b.ncells + 1)));
-    FIPI_CUDA(ctx, A((void**)&b.sp_keys, sizeof(unsigned) * 8 * n));
-    FIPI_CUDA(ctx, A((void**)&b.sp_keys_alt, sizeof(unsigned) * 8 * n));
-    FIPI_CUDA(ctx, A((void**)&b.sp_vals, sizeof(unsigned) * 8 * n));
-    FIPI_CUDA(ctx, A((void**)&b.sp_vals_alt, sizeof(unsigned) * 8 * n));
     FIPI_CUDA(ctx, A((void**)&b.sp_prev, sizeof(unsigned) * 8 * n));
     if (ctx->prec == FIPI_MIXED && b.n > 0) {
         FIPI_CUDA(ctx, A((void**)&b.sp_acc, sizeof(unsigned long long) * 4 * (size_t)P.nx * P.ny * P.nz));
     }
-    b.hist_cap = 256 * ((16 * n + RS_TILE - 1) / RS_TILE + 1);  // up to 16 records per particle (adjoint)
-    FIPI_CUDA(ctx, A((void**)&b.hist, sizeof(unsigned) * b.hist_cap));
+    if (ctx->prec == FIPI_FP64 && b.n > 0) {
+        const size_t V = (size_t)P.nx * P.ny * P.nz;
+        FIPI_CUDA(ctx, A((void**)&b.sp_head, sizeof(int) * V));
+        FIPI_CUDA(ctx, cudaMemsetAsync(b.sp_head, 0xff, sizeof(int) * V, ctx->stream));
+        FIPI_CUDA(ctx, A((void**)&b.sp_next, sizeof(int) * 8 * (size_t)n));
+    }
     FIPI_CUDA(ctx, A((void**)&b.tau_part, sizeof(double) * n));
     FIPI_CUDA(ctx, A((void**)&b.spos, sizeof(float4) * n));
     FIPI_CUDA(ctx, A((void**)&b.sp_fw, sizeof(double) * 6 * n));
@@ -1788,8 +1947,7 @@ fipi_status particles_alloc(fipi_ctx* ctx) {
 void particles_free(fipi_ctx* ctx) {
     ParticleBufs& b = ctx->pb;
     void* all[] = {b.p, b.p_old, b.u_old, b.f_pp, b.f_pi, b.r, b.cth, b.keys, b.keys_alt, b.ids, b.ids_alt,
-                   b.cell_off, b.cell_cnt, b.sp_keys, b.sp_keys_alt, b.sp_vals, b.sp_vals_alt, b.sp_prev,
-                   b.hist, b.tau_part, b.it_mark, b.tau, b.spos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
+                   b.cell_off, b.cell_cnt, b.sp_head, b.sp_next, b.sp_prev, b.tau_part, b.it_mark, b.tau, b.spos, b.sp_fw, b.ymax, b.sp_acc, b.uf, b.f_rand};
     for (void* p : all)
         if (p) cudaFree(p);
     b = ParticleBufs{};
@@ -2124,12 +2282,20 @@ fipi_status particles_spread_host(fipi_ctx* ctx, const double* p, const double* 
     if (st != FIPI_OK) return st;
     st = to_dev_soa(ctx, f_pp, fd, n);
     if (st != FIPI_OK) return st;
+    // lists of this call's own (the step's hold the previous spread's nodes);
+    // the FP64 form's heads are empty between spreads and shared
+    NodeLists nl{b.sp_head, ds.get<int>(8 * (size_t)n), ds.get<unsigned>(8 * (size_t)n)};
+    if (!nl.head) {
+        nl.head = ds.get<int>(V);
+        if (nl.head) FIPI_CUDA(ctx, cudaMemsetAsync(nl.head, 0xff, sizeof(int) * V, ctx->stream));
+    }
+    if (!nl.head || !nl.next || !nl.nodes) return set_error(ctx, FIPI_ERR_CUDA, "cudaMalloc failed");
     if (ctx->prec == FIPI_MIXED) {
         float* g = ds.get<float>(3 * V);
         if (!g) return set_error(ctx, FIPI_ERR_CUDA, "cudaMalloc failed");
         FIPI_CUDA(ctx, cudaMemsetAsync(g, 0, sizeof(float) * 3 * V, ctx->stream));
         float* f3[3] = {g, g + V, g + 2 * V};
-        spread_t<float>(ctx, pd, fd, f3, false);
+        spread_t<float>(ctx, pd, fd, f3, nl, false);
         std::vector<float> h(3 * V);
         FIPI_CUDA(ctx, cudaMemcpyAsync(h.data(), g, sizeof(float) * 3 * V, cudaMemcpyDeviceToHost, ctx->stream));
         FIPI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -2139,7 +2305,7 @@ fipi_status particles_spread_host(fipi_ctx* ctx, const double* p, const double* 
         if (!g) return set_error(ctx, FIPI_ERR_CUDA, "cudaMalloc failed");
         FIPI_CUDA(ctx, cudaMemsetAsync(g, 0, sizeof(double) * 3 * V, ctx->stream));
         double* f3[3] = {g, g + V, g + 2 * V};
-        spread_t<double>(ctx, pd, fd, f3, false);
+        spread_t<double>(ctx, pd, fd, f3, nl, false);
         FIPI_CUDA(ctx, cudaMemcpyAsync(out, g, sizeof(double) * 3 * V, cudaMemcpyDeviceToHost, ctx->stream));
         FIPI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
@@ -2156,6 +2322,16 @@ __global__ void k_set_tick(int* d_t, double* d_rmp, int t, double thr) {
 void set_tick(fipi_ctx* ctx, int t) {
     LaunchScope ls_(ctx, "step tick", 0.0);
     k_set_tick<<<1, 1, 0, ctx->stream>>>(ctx->d_t, ctx->d_rmp, t, 0.2 * ctx->P.t_end);
+}
+
+__global__ void k_set_ramp(double* rmp, int t, double thr) {
+    const double x = (double)(t + 1);
+    *rmp = (x < 0) ? 0.0 : (x < thr ? x / thr : 1.0);
+}
+
+void set_ramp(fipi_ctx* ctx, int t, double* rmp) {
+    LaunchScope ls_(ctx, "step tick", 0.0);
+    k_set_ramp<<<1, 1, 0, ctx->stream>>>(rmp, t, 0.2 * ctx->P.t_end);
 }
 
 // ------------------------------------------------------------ adjoint
@@ -2385,14 +2561,21 @@ __global__ void k_f_pp_adj(PC pc, const double* __restrict__ p, const unsigned* 
     }
 }
 
-// Spreading records of the interpolation adjoint: 8 corners of each of the
-// 2n interpolations (entity e = stage * n + i), node keys, fractions and
-// the 4 cotangents per entity.
-__global__ void k_adj_records(PC pc, const double* __restrict__ p0, const double* __restrict__ p1,
-                              const double* __restrict__ lamloc, unsigned* keys, unsigned* vals, double* rw) {
+// Records of the interpolation adjoint: 8 corners of each of the 2n
+// interpolations (entity e = stage * n + i) pushed onto the node lists,
+// fractions and the 4 cotangents per entity; with clear_prev `part` is zeroed
+// at the entity's nodes of the previous reversed step first.
+__global__ void k_adj_push(PC pc, const double* __restrict__ p0, const double* __restrict__ p1,
+                           const double* __restrict__ lamloc, NodeLists nl, double* rw, int clear_prev, double* part,
+                           size_t V) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = pc.n;
     if (e >= 2 * n) return;
+    if (clear_prev)
+        for (int c = 0; c < 8; ++c) {
+            const size_t nd = nl.nodes[8 * e + c];
+            for (int k = 0; k < 4; ++k) part[k * V + nd] = 0.0;
+        }
     const int st = e / n, i = e - st * n;
     const double* p = st == 0 ? p0 : p1;
     int ix[3];
@@ -2402,30 +2585,26 @@ __global__ void k_adj_records(PC pc, const double* __restrict__ p0, const double
         const int x = (ix[0] + c_corner[c][0]) % pc.N[0];
         const int y = (ix[1] + c_corner[c][1]) % pc.N[1];
         const int z = (ix[2] + c_corner[c][2]) % pc.N[2];
-        keys[8 * e + c] = (unsigned)(x + (size_t)y * pc.N[0] + (size_t)z * pc.N[0] * pc.N[1]);
-        vals[8 * e + c] = (unsigned)(8 * e + c);
+        push_record(nl, 8 * e + c, (unsigned)(x + (size_t)y * pc.N[0] + (size_t)z * pc.N[0] * pc.N[1]));
     }
     const int m = 2 * n;
     for (int a = 0; a < 3; ++a) rw[a * m + e] = fr[a];
     for (int q = 0; q < 4; ++q) rw[(3 + q) * m + e] = lamloc[(st * 4 + q) * n + i];
 }
 
-// Sorted segmented reduction of the records: part[q][node] = sum of w_c lam_q
-// in ascending record order (deterministic, no atomics).
-__global__ void k_adj_reduce(const unsigned* __restrict__ keys, const unsigned* __restrict__ vals, int m, int ne,
-                             const double* __restrict__ rw, double* part, size_t V) {
+// part[q][node] = sum of w_c lam_q in ascending record order.
+__global__ void k_adj_sum(NodeLists nl, int ne, const double* __restrict__ rw, double* part, size_t V) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= m) return;
-    const unsigned node = keys[s];
-    if (s > 0 && keys[s - 1] == node) return;
+    if (s >= 8 * ne) return;
+    const unsigned node = nl.nodes[s];
+    if (nl.head[node] != s) return;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = s; q < m && keys[q] == node; ++q) {
-        const unsigned rec = vals[q];
-        const int e = (int)(rec >> 3), c = (int)(rec & 7u);
+    owned_records(nl, s, node, [&](int rec) {
+        const int e = rec >> 3, c = rec & 7;
         const double o = rw[e], pp = rw[ne + e], qq = rw[2 * ne + e];
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc[k] += corner_value<double>(rw[(3 + k) * ne + e], c, o, pp, qq);
-    }
+    });
     for (int k = 0; k < 4; ++k) part[k * V + node] = acc[k];
 }
 
@@ -2470,8 +2649,8 @@ fipi_status particles_adjoint_alloc(fipi_ctx* ctx) {
     for (double** q : v1) FIPI_CUDA(ctx, A((void**)q, sizeof(double) * n));
     FIPI_CUDA(ctx, A((void**)&a.loc, sizeof(double) * 8 * n));
     FIPI_CUDA(ctx, A((void**)&a.lamloc, sizeof(double) * 8 * n));
-    unsigned** r16[] = {&a.rk, &a.rv, &a.rk2, &a.rv2};
-    for (unsigned** q : r16) FIPI_CUDA(ctx, A((void**)q, sizeof(unsigned) * 16 * n));
+    FIPI_CUDA(ctx, A((void**)&a.rnode, sizeof(unsigned) * 16 * n));
+    FIPI_CUDA(ctx, A((void**)&a.rnext, sizeof(int) * 16 * n));
     FIPI_CUDA(ctx, A((void**)&a.rw, sizeof(double) * 14 * n));
     FIPI_CUDA(ctx, A((void**)&a.rmp, sizeof(double)));
     return FIPI_OK;
@@ -2480,29 +2659,27 @@ fipi_status particles_adjoint_alloc(fipi_ctx* ctx) {
 void particles_adjoint_free(fipi_ctx* ctx) {
     AdjBufs& a = ctx->ad;
     void* all[] = {a.la_p, a.la_fpp, a.tp0, a.tfpp0, a.p1, a.fpi1, a.fpp1, a.lamF1, a.lamF2, a.lam_p1,
-                   a.loc, a.lamloc, a.rk, a.rv, a.rk2, a.rv2, a.rw, a.rmp, a.dct, a.pp_sig, a.pp_kn};
+                   a.loc, a.lamloc, a.rnode, a.rnext, a.rw, a.rmp, a.dct, a.pp_sig, a.pp_kn};
     for (void* p : all)
         if (p) cudaFree(p);
     a.la_p = a.la_fpp = a.tp0 = a.tfpp0 = a.p1 = a.fpi1 = a.fpp1 = a.lamF1 = a.lamF2 = a.lam_p1 = nullptr;
     a.dct = a.pp_sig = a.pp_kn = nullptr;
     a.loc = a.lamloc = a.rw = a.rmp = nullptr;
-    a.rk = a.rv = a.rk2 = a.rv2 = nullptr;
+    a.rnode = nullptr;
+    a.rnext = nullptr;
 }
 
-// Runs after the taped forward step: ctx->fb.c, fb.g hold c^{n+1}, grad c^{n+1};
-// a.tp0 holds p^n, a.rmp the ramp(t + 1, 0.2 t_end) factor of the reversed step.
+// a.in: the states before and after the reversed step; a.rmp: its
+// ramp(t + 1, 0.2 t_end) factor.
 fipi_status particles_adjoint(fipi_ctx* ctx) {
     ParticleBufs& b = ctx->pb;
     AdjBufs& a = ctx->ad;
     const PC pc = make_pc(ctx);
     const int n = b.n;
     const int nb = (n + 255) / 256;
-    const double* c = (const double*)ctx->fb.c;
-    const double* g0 = (const double*)ctx->fb.g[0];
-    const double* g1 = (const double*)ctx->fb.g[1];
-    const double* g2 = (const double*)ctx->fb.g[2];
+    const double *c = a.in.c1, *g0 = a.in.g1[0], *g1 = a.in.g1[1], *g2 = a.in.g1[2];
     // stage 1 recomputed at p^n: interpolation, f_pi, contact forces, p1
-    { LaunchScope ls_(ctx, "adjoint: interpolate + f_pi", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.tp0, c, g0, g1, g2, b.r, b.cth, a.loc, a.fpi1); }
+    { LaunchScope ls_(ctx, "adjoint: interpolate + f_pi", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.in.p0, c, g0, g1, g2, a.in.r, a.in.cth, a.loc, a.fpi1); }
     // the contact forces and their adjoint at positions q
     float4* spos = f_pp_path(ctx, false) != FppPath::cell ? b.spos : nullptr;
     auto contact_adj = [&](const double* q, const double* lamF, double* lam_p) {
@@ -2514,29 +2691,30 @@ fipi_status particles_adjoint(fipi_ctx* ctx) {
             k_f_pp_adj<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, q, b.ids, b.cell_off, a.rmp, lamF,
                                                                              lam_p, a.pp_kn);
     };
-    build_cells(ctx, a.tp0, false, spos);
-    f_pp_launch<double>(ctx, a.tp0, a.rmp, nullptr, a.fpp1, false, false, spos != nullptr);
-    { LaunchScope ls_(ctx, "adjoint: advect", 0.0); k_adj_advect1<<<nb, 256, 0, ctx->stream>>>(pc, a.tp0, a.fpi1, a.fpp1, b.r, a.p1); }
-    { LaunchScope ls_(ctx, "adjoint: interpolate", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.p1, c, g0, g1, g2, b.r, b.cth, a.loc + 4 * n, nullptr); }
+    build_cells(ctx, a.in.p0, false, spos);
+    f_pp_launch<double>(ctx, a.in.p0, a.rmp, nullptr, a.fpp1, false, false, spos != nullptr);
+    { LaunchScope ls_(ctx, "adjoint: advect", 0.0); k_adj_advect1<<<nb, 256, 0, ctx->stream>>>(pc, a.in.p0, a.fpi1, a.fpp1, a.in.r, a.p1); }
+    { LaunchScope ls_(ctx, "adjoint: interpolate", 0.0); k_adj_interp<<<nb, 256, 0, ctx->stream>>>(pc, a.p1, c, g0, g1, g2, a.in.r, a.in.cth, a.loc + 4 * n, nullptr); }
     // stage 2 reversed at p1
     // per-particle terms of this step's sigma (f_pi) and k_n cotangents
     FIPI_CUDA(ctx, cudaMemsetAsync(a.pp_sig, 0, sizeof(double) * n, ctx->stream));
     FIPI_CUDA(ctx, cudaMemsetAsync(a.pp_kn, 0, sizeof(double) * n, ctx->stream));
-    { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 2, a.p1, c, g0, g1, g2, a.loc + 4 * n, b.r, b.cth, a.la_p, a.la_fpp, nullptr, a.lamF2, a.lamloc + 4 * n, a.lam_p1, a.dct, a.pp_sig); }
+    { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 2, a.p1, c, g0, g1, g2, a.loc + 4 * n, a.in.r, a.in.cth, a.la_p, a.la_fpp, nullptr, a.lamF2, a.lamloc + 4 * n, a.lam_p1, a.dct, a.pp_sig); }
     build_cells(ctx, a.p1, false, spos);
     contact_adj(a.p1, a.lamF2, a.lam_p1);
     // stage 1 reversed at p^n (la_p becomes the start-state cotangent)
-    { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 1, a.tp0, c, g0, g1, g2, a.loc, b.r, b.cth, a.la_p, nullptr, a.lam_p1, a.lamF1, a.lamloc, a.la_p, a.dct, a.pp_sig); }
-    build_cells(ctx, a.tp0, false, spos);
-    contact_adj(a.tp0, a.lamF1, a.la_p);
+    { LaunchScope ls_(ctx, "adjoint: stage", 0.0); k_adj_stage<<<nb, 256, 0, ctx->stream>>>(pc, 1, a.in.p0, c, g0, g1, g2, a.loc, a.in.r, a.in.cth, a.la_p, nullptr, a.lam_p1, a.lamF1, a.lamloc, a.la_p, a.dct, a.pp_sig); }
+    build_cells(ctx, a.in.p0, false, spos);
+    contact_adj(a.in.p0, a.lamF1, a.la_p);
     param_acc(ctx, a.pp_sig, n, 1.0, a.pg + kPgSigmaAttach);
     param_acc(ctx, a.pp_kn, n, 1.0, a.pg + kPgKn);
     // interpolation adjoint onto the grid: part = [c, g0, g1, g2] cotangents
-    const int m = 16 * n;
-    { LaunchScope ls_(ctx, "adjoint: records", 0.0); k_adj_records<<<(2 * n + 255) / 256, 256, 0, ctx->stream>>>(pc, a.tp0, a.p1, a.lamloc, a.rk, a.rv, a.rw); }
-    radix_sort(ctx, a.rk, a.rv, a.rk2, a.rv2, m, bits_for(ctx->g.V - 1));
-    FIPI_CUDA(ctx, cudaMemsetAsync(a.part, 0, sizeof(double) * 4 * (size_t)ctx->g.V, ctx->stream));
-    { LaunchScope ls_(ctx, "adjoint: records reduce", 0.0); k_adj_reduce<<<(m + 255) / 256, 256, 0, ctx->stream>>>(a.rk, a.rv, m, 2 * n, a.rw, a.part, (size_t)ctx->g.V); }
+    const size_t V = (size_t)ctx->g.V;
+    const NodeLists nl{b.sp_head, a.rnext, a.rnode};
+    if (!a.part_valid) FIPI_CUDA(ctx, cudaMemsetAsync(a.part, 0, sizeof(double) * 4 * V, ctx->stream));
+    { LaunchScope ls_(ctx, "adjoint: records", 0.0); k_adj_push<<<(2 * n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, a.in.p0, a.p1, a.lamloc, nl, a.rw, a.part_valid ? 1 : 0, a.part, V); }
+    { LaunchScope ls_(ctx, "adjoint: record sums", 0.0); k_adj_sum<<<(16 * n + 127) / 128, 128, 0, ctx->stream>>>(nl, 2 * n, a.rw, a.part, V); }
+    a.part_valid = true;
     FIPI_CUDA(ctx, cudaGetLastError());
     return FIPI_OK;
 }
@@ -2546,7 +2724,7 @@ void particles_adjoint_spread(fipi_ctx* ctx) {
     const PC pc = make_pc(ctx);
     const int n = ctx->pb.n;
     LaunchScope ls_(ctx, "adjoint: spread", 0.0);
-    k_adj_spread<<<(n + 255) / 256, 256, 0, ctx->stream>>>(pc, a.tp0, a.tfpp0, a.lamF, (size_t)ctx->g.V, a.la_fpp, a.la_p);
+    k_adj_spread<<<(n + 255) / 256, 256, 0, ctx->stream>>>(pc, a.in.p0, a.in.fpp0, a.lamF, (size_t)ctx->g.V, a.la_fpp, a.la_p);
 }
 
 }  // namespace fipi
