@@ -381,6 +381,10 @@ template <typename T, int N, int COLS, int EM = FftE<T>::value> struct ZRtShape 
     // bank conflicts
     static constexpr bool WZ = RC == COLS && Tn <= 32 && THREADS >= 32 && FftPlan<N, EM>::NS >= 2;
     static constexpr int PAD = !WZ ? 0 : sizeof(T) == 4 ? 4 : 3;
+    // FP64 columns of up to 64 modes: four warps, so that the element-wise FP64
+    // work reaches all four FP64 pipes of an SM; the transforms take the first
+    // THREADS of them
+    static constexpr int BLOCK = sizeof(T) == 8 && WZ && THREADS < 128 ? 128 : THREADS;
     static constexpr int FSTRIDE = N * P + (PAD ? N >> PAD : 0);  // complex entries per field tile
 };
 // Z round-trip tile index: mode e of column c, with the pad slots.
@@ -401,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, NF == 1 && NB == 1 ? (sizeof(T) == 4
     using C = cplx<T>;
     constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     using SH = ZRtShape<T, N, COLS, EM>;
-    constexpr int RC = SH::RC, P = SH::P, NT = SH::THREADS;
+    constexpr int RC = SH::RC, P = SH::P, NT = SH::BLOCK;
     constexpr int ELEMS = COLS * N;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
@@ -451,11 +455,13 @@ __global__ void __launch_bounds__(kThreads, NF == 1 && NB == 1 ? (sizeof(T) == 4
             __syncthreads();
         }
         if constexpr (WZ && FX) {
-            C v[SH::E];
-            fx_fft_warp_column<DIR, N>(s + f * fstride, idx, wc, wt, twz, v);
-            using IOF = FftIO<T, DIR, N, EM>;
+            if (tid < SH::THREADS) {
+                C v[SH::E];
+                fx_fft_warp_column<DIR, N>(s + f * fstride, idx, wc, wt, twz, v);
+                using IOF = FftIO<T, DIR, N, EM>;
 #pragma unroll
-            for (int i = 0; i < SH::E; ++i) s[f * fstride + idx(wc, IOF::out_elem(wt, i))] = v[i];
+                for (int i = 0; i < SH::E; ++i) s[f * fstride + idx(wc, IOF::out_elem(wt, i))] = v[i];
+            }
         } else if constexpr (WZ) smem_fft2<T, DIR, N, EM, true>(s + f * fstride, idx, wc, wt, true, twz, 1);
         else
             for (int r = 0; r < COLS; r += RC) {
@@ -513,13 +519,14 @@ __global__ void __launch_bounds__(kThreads, NF == 1 && NB == 1 ? (sizeof(T) == 4
     if constexpr (WZ && FX) {
         // FP64: whole inverse transforms on the warps' columns, then full runs
         // from the tile
+        if (tid < SH::THREADS)
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            C v[SH::E];
-            fx_fft_warp_column<-DIR, N>(s + b * fstride, idx, wc, wt, twz, v);
+            for (int b = 0; b < NB; ++b) {
+                C v[SH::E];
+                fx_fft_warp_column<-DIR, N>(s + b * fstride, idx, wc, wt, twz, v);
 #pragma unroll
-            for (int i = 0; i < SH::E; ++i) s[b * fstride + idx(wc, IO::out_elem(wt, i))] = v[i];
-        }
+                for (int i = 0; i < SH::E; ++i) s[b * fstride + idx(wc, IO::out_elem(wt, i))] = v[i];
+            }
         __syncthreads();
 #pragma unroll
         for (int b = 0; b < NB; ++b)
@@ -738,11 +745,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_zpass_rr(Geom g, const tw_t<T>*
 // with 4-column tiles of all four outputs, 12 warps on an SM): 1261 -> 936 us at
 // 256^3 (three blocks of 85 registers an SM; 979 with two of 128).
 template <int NB, int DIR, int N, int COLS, class Op>
-__global__ void __launch_bounds__(ZRtShape<double, N, COLS>::THREADS, ZRtShape<double, N, COLS>::THREADS == kThreads ? 3 : 512 / ZRtShape<double, N, COLS>::THREADS)
+__global__ void __launch_bounds__(ZRtShape<double, N, COLS>::BLOCK, ZRtShape<double, N, COLS>::BLOCK == kThreads ? 3 : 4)
     k_zpass_rr_fx(Geom g, const longlong2* __restrict__ twz, Op op) {
     using C = double2;
     using SH = ZRtShape<double, N, COLS>;
-    constexpr int NT = SH::THREADS, ELEMS = COLS * N, E = SH::E, Tn = SH::Tn;
+    constexpr int NT = SH::BLOCK, ELEMS = COLS * N, E = SH::E, Tn = SH::Tn;
     using IOF = FftIO<double, DIR, N>;
     using IOI = FftIO<double, -DIR, N>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -759,10 +766,13 @@ __global__ void __launch_bounds__(ZRtShape<double, N, COLS>::THREADS, ZRtShape<d
     cp_async_commit();
     cp_async_wait_pending(1);
     __syncthreads();
+    const bool mine = tid < SH::THREADS;  // whole warps
     C v[E];
-    fx_fft_warp_column<DIR, N>(s, idx, wc, wt, twz, v);
+    if (mine) {
+        fx_fft_warp_column<DIR, N>(s, idx, wc, wt, twz, v);
 #pragma unroll
-    for (int i = 0; i < E; ++i) s[idx(wc, IOF::out_elem(wt, i))] = v[i];
+        for (int i = 0; i < E; ++i) s[idx(wc, IOF::out_elem(wt, i))] = v[i];
+    }
     cp_async_wait_all();
     __syncthreads();
     for (int e = tid; e < ELEMS; e += NT) {
@@ -774,20 +784,24 @@ __global__ void __launch_bounds__(ZRtShape<double, N, COLS>::THREADS, ZRtShape<d
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         FxSize size;
+        if (mine) {
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-            const int z = IOF::out_elem(wt, i);
-            typename Op::State st;
-            if (b == 0) st.f = v[i];
-            v[i] = op.rr_out(b, kx, ky0 + wc, z, st, sa[idx(wc, z)]);
-            size.add(v[i]);
+            for (int i = 0; i < E; ++i) {
+                const int z = IOF::out_elem(wt, i);
+                typename Op::State st;
+                if (b == 0) st.f = v[i];
+                v[i] = op.rr_out(b, kx, ky0 + wc, z, st, sa[idx(wc, z)]);
+                size.add(v[i]);
+            }
+            size = fx_row_size<Tn>(size);
         }
-        size = fx_row_size<Tn>(size);
         __syncthreads();  // the tile's previous contents are stored
-        fx_fft_regs<-DIR, N, true>(s, idx, wc, wt, true, twz, 1, size, v);
-        __syncwarp();
+        if (mine) {
+            fx_fft_regs<-DIR, N, true>(s, idx, wc, wt, true, twz, 1, size, v);
+            __syncwarp();
 #pragma unroll
-        for (int i = 0; i < E; ++i) s[idx(wc, IOI::out_elem(wt, i))] = v[i];
+            for (int i = 0; i < E; ++i) s[idx(wc, IOI::out_elem(wt, i))] = v[i];
+        }
         __syncthreads();
         for (int e = tid; e < ELEMS; e += NT) {
             const int c = e % COLS, z = e / COLS;

@@ -54,6 +54,7 @@ struct PC {
     // fixed-point sums with integer operations; positions stay FP64.
     double inv_d[3];   // 1/dx, 1/dy, 1/dz
     double inv_dc[3];  // 1/d_cell
+    double inv_pi, inv_mu;
     double mdc[3];     // margin/d_cell
     double drag;       // 6 pi mu: the Stokes drag is drag * r
     double img[3];     // d_cell (n_cell - 2): the minimum-image threshold
@@ -98,6 +99,8 @@ static PC make_pc(const fipi_ctx* ctx) {
         c.img[a] = c.dc[a] * (c.nc[a] - 2);
     }
     c.drag = 6.0 * c.pi * c.mu;
+    c.inv_pi = 1.0 / c.pi;
+    c.inv_mu = 1.0 / c.mu;
     c.f_req = (float)c.r_eq;
     c.f_req2 = c.f_req * c.f_req;
     c.inv_req2 = 1.0 / (c.r_eq * c.r_eq);
@@ -214,6 +217,19 @@ static int bits_for(long long maxval) {
     int b = 1;
     while ((1ll << b) <= maxval) ++b;
     return b;
+}
+
+// a / b with r = 1/b rounded to nearest at hand: the quotient estimate corrected
+// by its exact remainder is the correctly rounded quotient (P. Markstein, IBM J.
+// Res. Dev. 34, 1990), so the results are those of the division, in three
+// FP64 instructions instead of about ten.  Infinite, NaN and extreme values
+// (where the remainder would not be exact) take the division; b is finite and
+// not zero.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    const double q = a * r;
+    const int e = (__double2hiint(q) >> 20) & 0x7ff;  // between 2^-512 and 2^512: nothing under- or overflows
+    if ((unsigned)(e - 511) > 1024u) return (__double_as_longlong(a) << 1) == 0 ? q : a / b;
+    return fma(fma(-q, b, a), r, q);
 }
 
 // ------------------------------------------------------------ cell list
@@ -1107,9 +1123,10 @@ __device__ __forceinline__ int wrapi(int i, int n) {
 template <typename TF, typename TA>
 __device__ __forceinline__ void interp_fields(const PC& pc, double x, double y, double z, const TF* const* f, int nf,
                                               TA* out) {
-    const double fx = floor(x / pc.dx), fy = floor(y / pc.dy), fz = floor(z / pc.dz);
+    const double qx = div_by(x, pc.dx, pc.inv_d[0]), qy = div_by(y, pc.dy, pc.inv_d[1]), qz = div_by(z, pc.dz, pc.inv_d[2]);
+    const double fx = floor(qx), fy = floor(qy), fz = floor(qz);
     const int i = wrapi((int)fx, pc.N[0]), j = wrapi((int)fy, pc.N[1]), k = wrapi((int)fz, pc.N[2]);
-    const TA m = (TA)(x / pc.dx - fx), nn = (TA)(y / pc.dy - fy), o = (TA)(z / pc.dz - fz);
+    const TA m = (TA)(qx - fx), nn = (TA)(qy - fy), o = (TA)(qz - fz);
     const int i1 = (i + 1) % pc.N[0], j1 = (j + 1) % pc.N[1], k1 = (k + 1) % pc.N[2];
     for (int q = 0; q < nf; ++q) out[q] = interp<TF, TA>(f[q], i, j, k, i1, j1, k1, m, nn, o, pc.N[0], pc.N[1]);
 }
@@ -1145,9 +1162,10 @@ __device__ __forceinline__ void f_pi_of(const PC& pc, double phi, double gx, dou
         double f_mag;
         if (fabs(d) < r) f_mag = -pc.A * pc.pi * (d - r * ct) * pc.sigma;
         else f_mag = 0.0;
-        f[0] = gx / gn * f_mag;
-        f[1] = gy / gn * f_mag;
-        f[2] = gz / gn * f_mag;
+        const double ig = 1.0 / gn;
+        f[0] = div_by(gx, gn, ig) * f_mag;
+        f[1] = div_by(gy, gn, ig) * f_mag;
+        f[2] = div_by(gz, gn, ig) * f_mag;
     } else {
         f[0] = f[1] = f[2] = 0.0;
     }
@@ -1257,12 +1275,15 @@ __device__ __forceinline__ double wrap_exact(double x, double L) {
 __device__ __forceinline__ void advect_one(const PC& pc, int stage, const double* fpi, const double* fpp, double r,
                                            double* p, double* po, double* uo, const double* uf = nullptr,
                                            const double* fr = nullptr) {
+    const double ir = 1.0 / r;
     double v[3];
     for (int a = 0; a < 3; ++a) {
         double F = fpi[a] + 0.0;
         F = F + fpp[a];
         if (fr) F = F + fr[a];
-        v[a] = (uf ? uf[a] : 0.0) + F / 6.0 / pc.pi / pc.mu / r;
+        // F / 6 / pi / mu / r
+        F = div_by(div_by(div_by(div_by(F, 6.0, 1.0 / 6.0), pc.pi, pc.inv_pi), pc.mu, pc.inv_mu), r, ir);
+        v[a] = (uf ? uf[a] : 0.0) + F;
     }
     if (stage == 1) {
         for (int a = 0; a < 3; ++a) {
@@ -1445,13 +1466,12 @@ __global__ void k_stage_advect(PC pc, int stage, double* p, double* p_old, doubl
 __constant__ int c_corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {1, 0, 1}, {1, 1, 1}, {0, 0, 1}, {0, 1, 0}, {0, 1, 1}};
 
 __device__ __forceinline__ void cell_and_frac(const PC& pc, double X, double Y, double Z, int* ix, double* fr) {
-    const double fx = floor(X / pc.dx), fy = floor(Y / pc.dy), fz = floor(Z / pc.dz);
-    ix[0] = wrapi((int)fx, pc.N[0]);
-    ix[1] = wrapi((int)fy, pc.N[1]);
-    ix[2] = wrapi((int)fz, pc.N[2]);
-    fr[0] = X / pc.dx - fx;
-    fr[1] = Y / pc.dy - fy;
-    fr[2] = Z / pc.dz - fz;
+    const double q[3] = {div_by(X, pc.dx, pc.inv_d[0]), div_by(Y, pc.dy, pc.inv_d[1]), div_by(Z, pc.dz, pc.inv_d[2])};
+    for (int a = 0; a < 3; ++a) {
+        const double f = floor(q[a]);
+        ix[a] = wrapi((int)f, pc.N[a]);
+        fr[a] = q[a] - f;
+    }
 }
 
 // Spreading in ascending particle id without a sort.  Every record (particle
@@ -1565,7 +1585,7 @@ __global__ void k_spread_push(PC pc, const double* __restrict__ p, const double*
         push_record(nl, 8 * i + c, (unsigned)(x + (size_t)y * pc.N[0] + (size_t)z * pc.N[0] * pc.N[1]));
     }
     for (int a = 0; a < 3; ++a) {
-        fw[a * n + i] = (TA)((f_pp[a * n + i] + 0.0) / pc.dx / pc.dy / pc.dz);
+        fw[a * n + i] = (TA)div_by(div_by(div_by(f_pp[a * n + i] + 0.0, pc.dx, pc.inv_d[0]), pc.dy, pc.inv_d[1]), pc.dz, pc.inv_d[2]);
         fw[(3 + a) * n + i] = (TA)fr[a];
     }
 }
@@ -2343,9 +2363,10 @@ void set_ramp(fipi_ctx* ctx, int t, double* rmp) {
 // Trilinear value and position gradient of v at (x, y, z) (field.cpp:223-248).
 __device__ __forceinline__ void interp_grad(const PC& pc, double x, double y, double z, const double* __restrict__ v,
                                             double g[3]) {
-    const double fx = floor(x / pc.dx), fy = floor(y / pc.dy), fz = floor(z / pc.dz);
+    const double qx = div_by(x, pc.dx, pc.inv_d[0]), qy = div_by(y, pc.dy, pc.inv_d[1]), qz = div_by(z, pc.dz, pc.inv_d[2]);
+    const double fx = floor(qx), fy = floor(qy), fz = floor(qz);
     const int i = wrapi((int)fx, pc.N[0]), j = wrapi((int)fy, pc.N[1]), k = wrapi((int)fz, pc.N[2]);
-    const double m = x / pc.dx - fx, nn = y / pc.dy - fy, o = z / pc.dz - fz;
+    const double m = qx - fx, nn = qy - fy, o = qz - fz;
     const int i1 = (i + 1) % pc.N[0], j1 = (j + 1) % pc.N[1], k1 = (k + 1) % pc.N[2];
     const size_t sy = (size_t)pc.N[0], sz = (size_t)pc.N[0] * pc.N[1];
     const double v000 = v[i + j * sy + k * sz], v100 = v[i1 + j * sy + k * sz];
@@ -2358,9 +2379,9 @@ __device__ __forceinline__ void interp_grad(const PC& pc, double x, double y, do
                       (1 - m) * o * (v011 - v001) + m * o * (v111 - v101);
     const double dd = (1 - m) * (1 - nn) * (v001 - v000) + m * (1 - nn) * (v101 - v100) +
                       (1 - m) * nn * (v011 - v010) + m * nn * (v111 - v110);
-    g[0] = dm / pc.dx;
-    g[1] = dn / pc.dy;
-    g[2] = dd / pc.dz;
+    g[0] = div_by(dm, pc.dx, pc.inv_d[0]);
+    g[1] = div_by(dn, pc.dy, pc.inv_d[1]);
+    g[2] = div_by(dd, pc.dz, pc.inv_d[2]);
 }
 
 // Adjoint of f_pi_of: lf = cotangent of f_pi -> cotangents of phi and grad c,

@@ -505,11 +505,14 @@ template <typename T, int NF, int NT> struct XMinBlocks {
 // FP64 (block fixed point): for rows of 32 to 256 pairs the block is one field's
 // rows, so each row of every field belongs to one warp from the conversion to
 // the last (no idle lanes for an odd number of fields, no block barrier between
-// the transforms and the point loop); shorter rows share 256 threads.  The
+// the transforms and the point loop); shorter rows take the threads of all
+// fields' rows (32 x 256 x 128: c, f pass 166 us with 256 threads, most of them
+// idle, 35 with 32).  The
 // register budget follows what the tile leaves room for.  At 256^3 against 256
 // threads with block-wide rounds: c, f 407 -> 242 us, conv 640 -> 505, force
 // 1107 -> 955.
-template <int M> constexpr int x_fx_threads = M >= 32 ? x_rows_of(8, M) * FftPlan<M, 8>::Tn : kThreads;
+template <int M, int NF> constexpr int x_fx_threads =
+    M >= 32 ? x_rows_of(8, M) * FftPlan<M, 8>::Tn : (NF * x_rows_of(8, M) * FftPlan<M, 8>::Tn + 31) / 32 * 32;
 template <int NF, int NT> struct XMinBlocks<double, NF, NT> {
     static constexpr int at128 = NF <= 2 ? 5 : NF == 3 ? 4 : NF == 4 ? 3 : 2;
     static constexpr int value = at128 * 128 / NT > 0 ? at128 * 128 / NT : 1;
@@ -915,7 +918,7 @@ void launch_x(fipi_ctx* ctx, const char* name, int nreal, const Op& op, double* 
     dispatch_pow2<4, 256>(g.m, [&](auto MC) {
         constexpr int M = decltype(MC)::value;
         constexpr int TY = x_rows<T, M>;
-        constexpr int NT = sizeof(T) == sizeof(double) ? x_fx_threads<M> : kThreads;
+        constexpr int NT = sizeof(T) == sizeof(double) ? x_fx_threads<M, NF> : kThreads;
         const size_t smem = (size_t)NF * TY * xpass_pitch(g.m) * sizeof(cplx<T>);
         dim3 grid(g.ny / TY, g.nz);
         auto kern = k_xpass_acc<T, NIN, NOUT, REDUCE, M, Op, NT>;
@@ -1046,7 +1049,7 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
                 auto kern = k_zpass_rr_fx<NB, DIR, N, 2 * COLS, Op>;
                 static size_t granted = 48 * 1024;
                 ensure_smem(kern, smem, granted);
-                kern<<<dim3(g.h, g.ny / (2 * COLS)), SHF::THREADS, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
+                kern<<<dim3(g.h, g.ny / (2 * COLS)), SHF::BLOCK, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
             } else {
                 using SHP = ZRtShapeT<T, N, COLS, EM>;
                 constexpr int NS = NF > NB ? NF : NB;
@@ -1071,7 +1074,7 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
         auto kern = k_zpass_rt<T, NF, NB, DIR, N, CW, Op, EM>;
         static size_t granted = 48 * 1024;
         ensure_smem(kern, smem, granted);
-        kern<<<grid, SHP::THREADS, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
+        kern<<<grid, SHP::BLOCK, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
     });
 }
 
