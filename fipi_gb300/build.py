@@ -51,7 +51,6 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     OUT.mkdir(exist_ok=True)
     cc = nvcc()
     common = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-              "--split-compile", "0",  # optimise the units' kernels in parallel
               "-I", str(REPO / "include"), *(extra or [])]
     if verbose:
         common += ["-Xptxas", "-v"]
