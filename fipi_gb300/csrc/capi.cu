@@ -83,6 +83,16 @@ static void drain_timer(fipi_ctx* ctx) {
 
 using namespace fipi;
 
+// Step graphs with the particle work as a branch beside the grid passes.  The
+// particle kernels are chains of short launches; small grids leave SMs for
+// them and FP64 grid passes other pipes.  Particle stages beside the
+// projection, us a step without -> with: mixed 64^3 121 -> 111, 128^3 229 -> 213,
+// 256^3 1194 -> 1202 (the passes fill the SMs: mixed up to 2^21 nodes); FP64
+// 64^3 236 -> 206, 128^3 865 -> 820, 256^3 5686 -> 5463 (always).  Spreading beside
+// the Cahn-Hilliard part on top: mixed 64^3 111 -> 109, 128 x 128 x 64 159 -> 164,
+// 128^3 213 -> 280; FP64 64^3 206 -> 200, 128^3 820 -> 850 (up to 2^18 nodes).
+constexpr long long kBranchMixedMaxV = 1ll << 21, kBranchSpreadMaxV = 1ll << 18;
+
 static bool pow2_in(int n, int lo, int hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
 
 static fipi_status validate(const fipi_params* P, fipi_precision prec) {
@@ -205,6 +215,12 @@ fipi_status fipi_create(const fipi_params* P, fipi_precision prec, int device, f
     if (st != FIPI_OK) return fail(st);
     st = particles_alloc(ctx);
     if (st != FIPI_OK) return fail(st);
+    if (ctx->pb.n > 0 && P->switch_particle && (prec == FIPI_FP64 || ctx->g.V <= kBranchMixedMaxV)) {
+        e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
+        for (cudaEvent_t* ev : {&ctx->fork[0], &ctx->fork[1], &ctx->join[0], &ctx->join[1]})
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        if (e != cudaSuccess) return fail(cuda_check(ctx, e, "side stream"));
+    }
     if (ctx->pb.n > 0) {
         e = cudaMallocHost((void**)&ctx->pin, sizeof(double) * 12 * (size_t)ctx->pb.n);
         if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMallocHost(particle staging)"));
@@ -238,6 +254,9 @@ fipi_status fipi_destroy(fipi_ctx* ctx) {
     particles_free(ctx);
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    for (cudaEvent_t ev : {ctx->fork[0], ctx->fork[1], ctx->join[0], ctx->join[1]})
+        if (ev) cudaEventDestroy(ev);
     delete ctx;
     return FIPI_OK;
 }
@@ -499,9 +518,46 @@ void fipi::graphs_reset(fipi_ctx* ctx) {
 }
 
 
+// Runs f with the context stream replaced by the side stream, which waits for
+// the context stream's work so far (fork); the context stream waits for it in
+// join_branch.
+template <class F> static void on_branch(fipi_ctx* ctx, int k, F&& f) {
+    cudaEventRecord(ctx->fork[k], ctx->stream);
+    cudaStreamWaitEvent(ctx->side, ctx->fork[k], 0);
+    std::swap(ctx->stream, ctx->side);
+    f();
+    std::swap(ctx->stream, ctx->side);
+    cudaEventRecord(ctx->join[k], ctx->side);
+}
+static void join_branch(fipi_ctx* ctx, int k) { cudaStreamWaitEvent(ctx->stream, ctx->join[k], 0); }
+
 // One iteration of main.cpp:75-219, enqueued on the context stream.
-void fipi::enqueue_step(fipi_ctx* ctx) {
+//
+// With `branches` the particle stages (which read c and grad c) run beside the
+// projection (fluid coupling needs the projected velocity first) and, on the
+// smallest grids, the spreading (which reads the previous step's particles and
+// writes the spread grid) beside the Cahn-Hilliard part.
+void fipi::enqueue_step(fipi_ctx* ctx, bool branches) {
     const int t = ctx->t;
+    const bool parts = ctx->pb.n > 0 && ctx->P.switch_particle;
+    if (branches && parts) {
+        const bool early = ctx->g.V <= kBranchSpreadMaxV;
+        if (early) on_branch(ctx, 0, [&] { particles_spread(ctx); });
+        fields_step_ch(ctx, t);
+        if (early) join_branch(ctx, 0);
+        else particles_spread(ctx);
+        fields_step_force(ctx);
+        if (ctx->couple_u) {
+            fields_step_project(ctx);
+            particles_step(ctx);
+        } else {
+            on_branch(ctx, 1, [&] { particles_step(ctx); });
+            fields_step_project(ctx);
+            join_branch(ctx, 1);
+        }
+        ctx->t = t + 1;
+        return;
+    }
     fields_step_ch(ctx, t);      // main.cpp:79-141
     particles_spread(ctx);       // main.cpp:169 (compute_f_r of the previous step's state)
     fields_step_stokes(ctx);     // main.cpp:146-181
@@ -533,7 +589,7 @@ static fipi_status graph_step(fipi_ctx* ctx, bool* done) {
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            enqueue_step(ctx);
+            enqueue_step(ctx, ctx->side != nullptr);
             e = cudaStreamEndCapture(ctx->stream, &graph);
         }
         cudaGraphExec_t exec = nullptr;

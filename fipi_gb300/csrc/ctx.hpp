@@ -210,6 +210,8 @@ struct fipi_ctx {
         long long launches = 0;
     } graphs[2];
     bool use_graphs = true;
+    cudaStream_t side = nullptr;  // second branch of the step graph (small grids)
+    cudaEvent_t fork[2] = {}, join[2] = {};
     int substep = 0;           // 1 after fipi_step_ch, 2 after fipi_step_stokes
     double* pin = nullptr;     // pinned host staging of the particle state, 12 n doubles
     double* pin_dev = nullptr; // the same buffer as a device pointer (mapped pinned memory)
@@ -244,7 +246,9 @@ fipi_status fields_get_phase(fipi_ctx* ctx, double* c, bool dev = false);
 fipi_status fields_get_velocity(fipi_ctx* ctx, double* u, bool dev = false);
 // The three grid sub-steps of one iteration (enqueue only).
 void fields_step_ch(fipi_ctx* ctx, int t);        // conv, CH update, c, f
-void fields_step_stokes(fipi_ctx* ctx);           // mu, grad c, force, projection
+void fields_step_stokes(fipi_ctx* ctx);           // mu, grad c, force, projection: the two below
+void fields_step_force(fipi_ctx* ctx);            // mu, grad c (stored), force and its X transform
+void fields_step_project(fipi_ctx* ctx);          // the rest of its transform, projection
 fipi_status fields_get_grad(fipi_ctx* ctx, double* g_host);  // grad c of the state, 3 x V
 fipi_status fields_mass(fipi_ctx* ctx, double* out);
 fipi_status fields_free_energy(fipi_ctx* ctx, double* out);
@@ -293,7 +297,9 @@ fipi_status particles_get_radii(fipi_ctx* ctx, double* r_host);
 fipi_status particles_wrap(fipi_ctx* ctx, double* p_host);
 
 // Reverse mode (adjoint.cu / particles.cu).
-void enqueue_step(fipi_ctx* ctx);  // one forward step, direct launches
+// One forward step; `branches`: with the particle work on ctx->side where
+// nothing orders it behind the grid work (step graphs of small grids).
+void enqueue_step(fipi_ctx* ctx, bool branches = false);
 // Sets the device step index and the ramp factor of step t (particles.cu).
 void set_tick(fipi_ctx* ctx, int t);
 // *rmp = ramp(t + 1, 0.2 t_end).
