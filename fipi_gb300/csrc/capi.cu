@@ -207,6 +207,8 @@ fipi_status fipi_create(const fipi_params* P, fipi_precision prec, int device, f
     if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaStreamCreate"));
     e = cudaMalloc(&ctx->status, sizeof(int));
     if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMalloc(status)"));
+    e = cudaMallocHost((void**)&ctx->status_pin, sizeof(int));
+    if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMallocHost(status)"));
     e = cudaMalloc(&ctx->d_t, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rmp, sizeof(double));
     if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMalloc(step counter)"));
@@ -215,12 +217,6 @@ fipi_status fipi_create(const fipi_params* P, fipi_precision prec, int device, f
     if (st != FIPI_OK) return fail(st);
     st = particles_alloc(ctx);
     if (st != FIPI_OK) return fail(st);
-    if (ctx->pb.n > 0 && P->switch_particle && (prec == FIPI_FP64 || ctx->g.V <= kBranchMixedMaxV)) {
-        e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
-        for (cudaEvent_t* ev : {&ctx->fork[0], &ctx->fork[1], &ctx->join[0], &ctx->join[1]})
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-        if (e != cudaSuccess) return fail(cuda_check(ctx, e, "side stream"));
-    }
     if (ctx->pb.n > 0) {
         e = cudaMallocHost((void**)&ctx->pin, sizeof(double) * 12 * (size_t)ctx->pb.n);
         if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMallocHost(particle staging)"));
@@ -253,6 +249,7 @@ fipi_status fipi_destroy(fipi_ctx* ctx) {
     fields_free(ctx);
     particles_free(ctx);
     if (ctx->status) cudaFree(ctx->status);
+    if (ctx->status_pin) cudaFreeHost(ctx->status_pin);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     for (cudaEvent_t ev : {ctx->fork[0], ctx->fork[1], ctx->join[0], ctx->join[1]})
@@ -272,9 +269,11 @@ fipi_status fipi_device_bytes(const fipi_ctx* ctx, size_t* out) {
 fipi_status fipi::check_status(fipi_ctx* ctx) {
     // the copy of the error word is ordered after all enqueued work, so one
     // synchronisation covers both
-    int st = 0;
-    FIPI_CUDA(ctx, d2h(ctx, &st, ctx->status, sizeof(int)));
+    // (pinned: a copy to pageable memory goes through a staging buffer of the
+    // driver's)
+    FIPI_CUDA(ctx, d2h(ctx, ctx->status_pin, ctx->status, sizeof(int)));
     FIPI_CUDA(ctx, cudaGetLastError());
+    const int st = *ctx->status_pin;
     if (st) {
         FIPI_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
         if (st & ERR_TMA_TIMEOUT) return set_error(ctx, FIPI_ERR_TIMEOUT, "a bulk-copy wait timed out in an FFT pass");
@@ -295,12 +294,7 @@ static fipi_status set_phase_impl(fipi_ctx* ctx, const double* c, bool dev) {
     fipi_status st = fields_set_phase(ctx, c, dev);
     if (st != FIPI_OK) return st;
     ctx->t = 0;
-    // device step counter and ramp(t + 1, 0.2 t_end) for t = 0
-    const int t0 = 0;
-    const double thr = 0.2 * ctx->P.t_end;
-    const double rmp = (1.0 < thr) ? 1.0 / thr : 1.0;
-    FIPI_CUDA(ctx, h2d(ctx, ctx->d_t, &t0, sizeof(int)));
-    FIPI_CUDA(ctx, h2d(ctx, ctx->d_rmp, &rmp, sizeof(double)));
+    set_tick(ctx, 0);  // device step counter and ramp(1, 0.2 t_end)
     ctx->have_phase = true;
     return check_status(ctx);
 }
@@ -587,6 +581,12 @@ static fipi_status graph_step(fipi_ctx* ctx, bool* done) {
         const int t0 = ctx->t;
         const long long l0 = ctx->kt.launches;
         cudaGraph_t graph = nullptr;
+        if (!ctx->side && ctx->pb.n > 0 && ctx->P.switch_particle &&
+            (ctx->prec == FIPI_FP64 || ctx->g.V <= kBranchMixedMaxV)) {
+            FIPI_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+            for (cudaEvent_t* ev : {&ctx->fork[0], &ctx->fork[1], &ctx->join[0], &ctx->join[1]})
+                FIPI_CUDA(ctx, cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+        }
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             enqueue_step(ctx, ctx->side != nullptr);

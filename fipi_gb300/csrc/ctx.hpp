@@ -14,6 +14,7 @@ namespace fipi {
 
 // Device buffers of one precision form.  T = float (mixed) or double.
 struct FieldBufs {
+    void* tables = nullptr;  // the tables below
     void* twx = nullptr;  // exp(-2 pi i q / nx), q < nx     (cplx<T>)
     void* twy = nullptr;  // exp(-2 pi i q / ny)
     void* twz = nullptr;  // exp(-2 pi i q / nz)
@@ -196,6 +197,7 @@ struct fipi_ctx {
     double* partials = nullptr;  // per-block FP64 partial sums
     int n_partials = 0;
     int* status = nullptr;       // device error word
+    int* status_pin = nullptr;   // its pinned host copy (check_status)
     double* scratch_d = nullptr; // small FP64 device scratch (reductions)
     int t = 0;
     int* d_t = nullptr;          // device copy of t (advanced by step_tick or the last advection)

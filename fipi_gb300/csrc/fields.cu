@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstring>
+#include <utility>
 #include <vector>
 
 #include "ctx.hpp"
@@ -569,12 +571,6 @@ template <typename T> static fipi_status alloc_fields_t(fipi_ctx* ctx) {
         if (e == cudaSuccess) ctx->device_bytes += bytes;
         return e;
     };
-    FIPI_CUDA(ctx, A(&b.twx, sizeof(C) * g.nx));
-    FIPI_CUDA(ctx, A(&b.twy, sizeof(C) * g.ny));
-    FIPI_CUDA(ctx, A(&b.twz, sizeof(C) * g.nz));
-    FIPI_CUDA(ctx, A(&b.kx, sizeof(T) * (g.m + 1)));
-    FIPI_CUDA(ctx, A(&b.ky, sizeof(T) * g.ny));
-    FIPI_CUDA(ctx, A(&b.kz, sizeof(T) * g.nz));
     FIPI_CUDA(ctx, A(&b.c, sizeof(T) * V));
     for (int d = 0; d < 3; ++d) {
         FIPI_CUDA(ctx, A(&b.g[d], sizeof(T) * V));
@@ -589,48 +585,58 @@ template <typename T> static fipi_status alloc_fields_t(fipi_ctx* ctx) {
         FIPI_CUDA(ctx, A(p, sizeof(C) * SH));
         FIPI_CUDA(ctx, cudaMemsetAsync(*p, 0, sizeof(C) * SH, ctx->stream));
     }
-    // twiddles and wave numbers, computed in extended precision on the host
-    auto twiddles = [&](int n) {
-        std::vector<C> t(n);
-        const long double two_pi = 6.283185307179586476925286766559005768L;
-        for (int q = 0; q < n; ++q) {
-            const long double a = two_pi * (long double)q / (long double)n;
-            t[q].x = (T)cosl(a);
-            t[q].y = (T)(-sinl(a));
-        }
-        return t;
+    // twiddles and wave numbers, computed in extended precision on the host:
+    // one table per axis length, all in one allocation and one copy
+    std::vector<unsigned char> blob;
+    std::vector<std::pair<void**, size_t>> at;  // where each table's pointer goes, offset in the blob
+    auto put = [&](void** dst, const void* src, size_t bytes) {
+        const size_t o = (blob.size() + 255) & ~(size_t)255;
+        blob.resize(o + bytes);
+        std::memcpy(blob.data() + o, src, bytes);
+        at.push_back({dst, o});
     };
-    auto tx = twiddles(g.nx), ty = twiddles(g.ny), tz = twiddles(g.nz);
-    FIPI_CUDA(ctx, h2d(ctx, b.twx, tx.data(), sizeof(C) * g.nx));
-    FIPI_CUDA(ctx, h2d(ctx, b.twy, ty.data(), sizeof(C) * g.ny));
-    FIPI_CUDA(ctx, h2d(ctx, b.twz, tz.data(), sizeof(C) * g.nz));
-    if constexpr (sizeof(T) == sizeof(double)) {  // block fixed-point factors (fx64.cuh)
-        auto factors = [&](void** dst, int n) -> cudaError_t {
-            std::vector<longlong2> t(n);
-            const long double two_pi = 6.283185307179586476925286766559005768L, one = 4611686018427387904.0L;
+    std::vector<std::pair<long double, long double>> cs;  // cos, sin of 2 pi q / cs.size()
+    auto twiddles = [&](int n, void** tw, void** fw) {
+        if ((int)cs.size() != n) {
+            cs.resize(n);
+            const long double two_pi = 6.283185307179586476925286766559005768L;
             for (int q = 0; q < n; ++q) {
                 const long double a = two_pi * (long double)q / (long double)n;
-                t[q].x = fx_pack(llrintl(cosl(a) * one));
-                t[q].y = fx_pack(llrintl(-sinl(a) * one));
+                cs[q] = {cosl(a), sinl(a)};
             }
-            const cudaError_t e = A(dst, sizeof(longlong2) * n);
-            return e != cudaSuccess ? e : h2d(ctx, *dst, t.data(), sizeof(longlong2) * n);
-        };
-        FIPI_CUDA(ctx, factors(&b.fwx, g.nx));
-        FIPI_CUDA(ctx, factors(&b.fwy, g.ny));
-        FIPI_CUDA(ctx, factors(&b.fwz, g.nz));
-    }
+        }
+        std::vector<C> t(n);
+        for (int q = 0; q < n; ++q) {
+            t[q].x = (T)cs[q].first;
+            t[q].y = (T)(-cs[q].second);
+        }
+        put(tw, t.data(), sizeof(C) * n);
+        if constexpr (sizeof(T) == sizeof(double)) {  // block fixed-point factors (fx64.cuh)
+            std::vector<longlong2> f(n);
+            const long double one = 4611686018427387904.0L;
+            for (int q = 0; q < n; ++q) {
+                f[q].x = fx_pack(llrintl(cs[q].first * one));
+                f[q].y = fx_pack(llrintl(-cs[q].second * one));
+            }
+            put(fw, f.data(), sizeof(longlong2) * n);
+        }
+    };
+    twiddles(g.nx, &b.twx, &b.fwx);
+    twiddles(g.ny, &b.twy, &b.fwy);
+    twiddles(g.nz, &b.twz, &b.fwz);
     // field.cpp:100-121: i*2.0*pi/L for i <= N/2 else (i - N)*2.0*pi/L
     const fipi_params& P = ctx->P;
-    auto waves = [&](int n, int count, double L) {
+    auto waves = [&](void** dst, int n, int count, double L) {
         std::vector<T> k(count);
         for (int i = 0; i < count; ++i) k[i] = (T)((i <= n / 2) ? i * 2.0 * P.pi / L : (i - n) * 2.0 * P.pi / L);
-        return k;
+        put(dst, k.data(), sizeof(T) * count);
     };
-    auto kx = waves(g.nx, g.m + 1, P.lx), ky = waves(g.ny, g.ny, P.ly), kz = waves(g.nz, g.nz, P.lz);
-    FIPI_CUDA(ctx, h2d(ctx, b.kx, kx.data(), sizeof(T) * (g.m + 1)));
-    FIPI_CUDA(ctx, h2d(ctx, b.ky, ky.data(), sizeof(T) * g.ny));
-    FIPI_CUDA(ctx, h2d(ctx, b.kz, kz.data(), sizeof(T) * g.nz));
+    waves(&b.kx, g.nx, g.m + 1, P.lx);
+    waves(&b.ky, g.ny, g.ny, P.ly);
+    waves(&b.kz, g.nz, g.nz, P.lz);
+    FIPI_CUDA(ctx, A(&b.tables, blob.size()));
+    for (auto& x : at) *x.first = (unsigned char*)b.tables + x.second;
+    FIPI_CUDA(ctx, h2d(ctx, b.tables, blob.data(), blob.size()));
     return FIPI_OK;
 }
 
@@ -660,7 +666,7 @@ fipi_status fields_alloc(fipi_ctx* ctx) {
 
 void fields_free(fipi_ctx* ctx) {
     FieldBufs& b = ctx->fb;
-    void* all[] = {b.twx, b.twy, b.twz, b.fwx, b.fwy, b.fwz, b.kx, b.ky, b.kz, b.c, b.ureal, b.chat, b.chat_old, b.fhat,
+    void* all[] = {b.tables, b.c, b.ureal, b.chat, b.chat_old, b.fhat,
                    b.fhat_old, b.Chat_old, b.S[0], b.S[1], b.S[2], b.S[3], b.g[0], b.g[1], b.g[2],
                    b.fsp[0], b.fsp[1], b.fsp[2], b.upre[0], b.upre[1], b.upre[2], ctx->partials, ctx->k0};
     for (void* p : all)
@@ -692,8 +698,7 @@ template <typename T> static fipi_status store_real(fipi_ctx* ctx, const T* src,
         LaunchScope ls(ctx, "convert", 0.0);
         k_convert<T, double><<<1024, 256, 0, ctx->stream>>>(src, dst, n);
     }
-    FIPI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return FIPI_OK;
+    return FIPI_OK;  // the caller's check_status waits
 }
 
 // Compensated (Neumaier) FP64 sum of device values in a fixed order:
@@ -801,13 +806,37 @@ fipi_status fields_get_phase(fipi_ctx* ctx, double* c, bool dev) {
     return store_real<double>(ctx, (const double*)ctx->fb.c, c, (size_t)ctx->g.V, dev);
 }
 
-// Real velocity u (3 x V) into fb.ureal from the velocity state.
-template <typename T> static void velocity_real_t(fipi_ctx* ctx) {
+// C2R of three fields into FP64 arrays (the mixed form's velocity read into a
+// caller's device array: no FP32 copy in between).
+struct OpC2RStoreWide {
+    const float2* src[3];
+    double* dst;
+    size_t V;
+    int nx, ny;
+    __device__ const float2* in(int f) const { return src[f]; }
+    __device__ float2* out(int) const { return nullptr; }
+    __device__ void point(int z, int y, int n, float2* v) const {
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            reinterpret_cast<double2*>(dst + f * V + ((size_t)z * ny + y) * nx)[n] = make_double2(v[f].x, v[f].y);
+    }
+};
+
+// Real velocity u (3 x V) into fb.ureal, or with `wide` into that FP64 device
+// array, from the velocity state.
+template <typename T> static void velocity_real_t(fipi_ctx* ctx, double* wide = nullptr) {
     const Geom& g = ctx->g;
     void* up[3] = {ctx->fb.upre[0], ctx->fb.upre[1], ctx->fb.upre[2]};
     void* sp[3] = {ctx->fb.S[0], ctx->fb.S[1], ctx->fb.S[2]};
     launch_y<T>(ctx, 3, up, sp, +1);
-    T* ur = (T*)ctx->fb.ureal;
+    if constexpr (sizeof(T) == sizeof(float)) {
+        if (wide) {
+            OpC2RStoreWide op{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, wide, (size_t)g.V, g.nx, g.ny};
+            launch_x<T, 3, 0, false>(ctx, "X inverse store", 6, NoAcc<OpC2RStoreWide>{op});
+            return;
+        }
+    }
+    T* ur = wide ? (T*)wide : (T*)ctx->fb.ureal;
     OpC2RStore<T, 3> op{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, {ur, ur + g.V, ur + 2 * g.V}, g.nx, g.ny};
     launch_x<T, 3, 0, false>(ctx, "X inverse store", 3, NoAcc<OpC2RStore<T, 3>>{op});
 }
@@ -818,8 +847,11 @@ void fields_velocity_real(fipi_ctx* ctx) {
 }
 
 template <typename T> static fipi_status get_velocity_t(fipi_ctx* ctx, double* u, bool dev) {
-    velocity_real_t<T>(ctx);
+    // (vector stores need a 16-byte aligned destination)
+    const bool direct = dev && (uintptr_t)u % 16 == 0;
+    velocity_real_t<T>(ctx, direct ? u : nullptr);
     FIPI_CUDA(ctx, cudaGetLastError());
+    if (direct) return FIPI_OK;  // the caller's check_status waits
     return store_real<T>(ctx, (T*)ctx->fb.ureal, u, (size_t)ctx->g.V * 3, dev);
 }
 
