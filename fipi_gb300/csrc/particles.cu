@@ -824,8 +824,8 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
 // d_cell).  About one candidate in twelve lies within r_eq (4/3 pi r_eq^3
 // against 27 cells), so these separations only select: candidates within
 // r_eq plus their rounding bound (f_req2_sel) are queued by ballot, and every
-// 32 of them are evaluated with all lanes busy, in FP64 from the FP64
-// positions with the minimum-image rule of cluster.cpp:225-232 (shift d by L
+// 32 of them are evaluated with all lanes busy, from FP64 separations
+// with the minimum-image rule of cluster.cpp:225-232 (shift d by L
 // when |d| exceeds d_cell (n_cell - 2)).  FP64 issues at 1/64 of the FP32 rate:
 // 40 pairs a particle instead of 500.  The selection sees the same image as
 // the rule for every pair that
@@ -929,7 +929,8 @@ __device__ __forceinline__ double inv_distance(double s) {
 }
 
 // Queues the staged candidates of home particle i (at h in the home frame)
-// and calls body(id) with full warps of them; `held` candidates stay queued.
+// and calls body(id) with full warps of them; `held` candidates stay queued
+// (the caller passes them on last, -1 for the lanes left over).
 template <class Body>
 __device__ __forceinline__ void fpp_select(const PC& pc, const FppShared& sh, int* queue, float4 h, int count, int lane,
                                            int& held, Body&& body) {
@@ -987,12 +988,17 @@ __device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict
                 }
                 if (on) fpp_select(pc, sh, sh.queue[w], h, count, lane, held, pair);
             }
-            if (lane < held) pair(sh.queue[w][lane]);
+            if (held > 0) pair(lane < held ? sh.queue[w][lane] : -1);
             __syncwarp();
         });
     }
 }
 
+// TA: the arithmetic the forces are formed and summed in (k_f_pp's): double in
+// the FP64 form; float in the mixed form, from the FP64 separations and added
+// one after the other in the reference's pair order, so that the mixed form's
+// forces are k_f_pp<float>'s bit for bit.
+template <typename TA>
 __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const double* __restrict__ p,
                                                               const float4* __restrict__ spos,
                                                               const int* __restrict__ off,
@@ -1009,33 +1015,65 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const doubl
     fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
         const int i = __float_as_int(h.w);
         const bool tau_on = mark && any_force(f_pi, n, i);
-        double ax = 0.0, ay = 0.0, az = 0.0, tau = 0.0;
         const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
-        const double str = *rmp_p * pc.k_n;
+        const double rmp = *rmp_p, str = rmp * pc.k_n;
+        TA ax = TA(0), ay = TA(0), az = TA(0);
+        double tau = 0.0;
         walk([&](int j) {
-            double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
-                           min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
-            double d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
-            if (!nonzero_bits(d2) && !nonzero_bits(d[0]) && !nonzero_bits(d[1]) && !nonzero_bits(d[2])) {
-                coincident_d(min(i, j), max(i, j), pc.r_p, d);
-                if (j < i)
-                    for (int a = 0; a < 3; ++a) d[a] = -d[a];
-                d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+            double d[3] = {0.0, 0.0, 0.0}, d2 = 0.0;
+            if (j >= 0) {
+                d[0] = min_image(xi - p[j], pc.img[0], pc.L[0]);
+                d[1] = min_image(yi - p[n + j], pc.img[1], pc.L[1]);
+                d[2] = min_image(zi - p[2 * n + j], pc.img[2], pc.L[2]);
+                if (!nonzero_bits(d[0]) && !nonzero_bits(d[1]) && !nonzero_bits(d[2])) {
+                    coincident_d(min(i, j), max(i, j), pc.r_p, d);
+                    if (j < i)
+                        for (int a = 0; a < 3; ++a) d[a] = -d[a];
+                }
             }
-            // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
-            const double y = inv_distance(d2 * pc.inv_req2);
-            const long long yb = __double_as_longlong(y);
-            if (yb <= 0x3ff0000000000000ll || yb > 0x7ff0000000000000ll) return;  // !(y > 1), on the bits
-            const double sc = fma(y, str, -str);
-            ax = fma(d[0], sc, ax);
-            ay = fma(d[1], sc, ay);
-            az = fma(d[2], sc, az);
-            if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
+            if constexpr (sizeof(TA) == sizeof(float)) {
+                const float dx = (float)d[0], dy = (float)d[1], dz = (float)d[2];
+                const float dn = sqrtf(dx * dx + dy * dy + dz * dz);
+                const bool in = j >= 0 && dn < (float)pc.r_eq;
+                const float sc = ((float)pc.r_eq - dn) * (float)rmp * (float)pc.k_n;
+                const float fx = (dx / dn) * sc, fy = (dy / dn) * sc, fz = (dz / dn) * sc;
+                if (in && tau_on && i < j)
+                    tau += (double)fx * 0.5 * d[0] + (double)fy * 0.5 * d[1] + (double)fz * 0.5 * d[2];
+                for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
+                    const int l = __ffs(m) - 1;
+                    ax += __shfl_sync(0xffffffffu, fx, l);
+                    ay += __shfl_sync(0xffffffffu, fy, l);
+                    az += __shfl_sync(0xffffffffu, fz, l);
+                }
+            } else {
+                if (j < 0) return;
+                d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+                // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
+                const double y = inv_distance(d2 * pc.inv_req2);
+                const long long yb = __double_as_longlong(y);
+                if (yb <= 0x3ff0000000000000ll || yb > 0x7ff0000000000000ll) return;  // !(y > 1), on the bits
+                const double sc = fma(y, str, -str);
+                ax = fma(d[0], sc, ax);
+                ay = fma(d[1], sc, ay);
+                az = fma(d[2], sc, az);
+                if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
+            }
         });
-        const double t = warp_total4(ax, ay, az, tau, lane);
-        if (on && (lane & 7) == 0) {
-            if (lane < 24) f_pp[(lane >> 3) * n + i] = t;
-            else if (tau_part) tau_part[i] = t;
+        if constexpr (sizeof(TA) == sizeof(float)) {  // every lane holds the sums
+            if (tau_on)
+                for (int o = 16; o > 0; o >>= 1) tau += __shfl_xor_sync(0xffffffffu, tau, o);
+            if (on && lane == 0) {
+                f_pp[i] = (double)ax;
+                f_pp[n + i] = (double)ay;
+                f_pp[2 * n + i] = (double)az;
+                if (tau_part) tau_part[i] = tau;
+            }
+        } else {
+            const double t = warp_total4(ax, ay, az, tau, lane);
+            if (on && (lane & 7) == 0) {
+                if (lane < 24) f_pp[(lane >> 3) * n + i] = t;
+                else if (tau_part) tau_part[i] = t;
+            }
         }
     });
 }
@@ -1776,7 +1814,7 @@ static void it_mark_launch(fipi_ctx* ctx, const double* p) {
 // minimum image (see there); otherwise (margin != 0, or 3 cells on an axis and
 // r_eq > d_cell) k_f_pp, one warp per home cell in the reference's pair order.
 // Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp 110;
-// 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 16; mixed, 20,000
+// 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 21; mixed, 20,000
 // particles, k_f_pp_fast 27.
 enum class FppPath { cell, warp, fast };
 static FppPath f_pp_path(const fipi_ctx* ctx, bool fp32) {
@@ -1802,7 +1840,7 @@ static void f_pp_launch(fipi_ctx* ctx, const double* p, const double* rmp, const
             k_f_pp_fast<<<b.ncells, 32 * kFppRows, 0, ctx->stream>>>(pc, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr,
                                                                      b.it_mark, f_pp, tau ? b.tau_part : nullptr);
         else
-            k_f_pp_warp<<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
+            k_f_pp_warp<TA><<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
                 pc, p, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp,
                 tau ? b.tau_part : nullptr);
     } else {
@@ -2532,6 +2570,7 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_adj_warp(PC pc, const d
         const double li[3] = {lamF[i], lamF[n + i], lamF[2 * n + i]};
         double acc[3] = {0.0, 0.0, 0.0}, acc_kn = 0.0;
         walk([&](int j) {
+            if (j < 0) return;
             const double d[3] = {min_image(xi - p[j], pc.img[0], pc.L[0]), min_image(yi - p[n + j], pc.img[1], pc.L[1]),
                                  min_image(zi - p[2 * n + j], pc.img[2], pc.L[2])};
             pair_adj(pc, d, li, lamF, j, rmp, acc, acc_kn);
