@@ -371,7 +371,12 @@ __global__ void __launch_bounds__(kThreads) k_zpass(Geom g, const tw_t<T>* __res
 template <typename T, int N, int COLS, int EM = FftE<T>::value> struct ZRtShape {
     static constexpr int E = N < EM ? N : EM;
     static constexpr int Tn = N / E;                                      // threads per column FFT
-    static constexpr int RC = COLS * Tn <= kThreads ? COLS : kThreads / Tn;  // columns per FFT round
+    // FP32 columns of 512 modes: blocks of 512 threads keep 16 columns (128-byte
+    // runs) and a warp per column; with 256 threads the CH update ran its columns
+    // in two rounds and the projection 8-column tiles (512^3: 1026 -> 931 us and
+    // 1988 -> 1745)
+    static constexpr int CAP = sizeof(T) == 4 && N == 512 ? 512 : kThreads;
+    static constexpr int RC = COLS * Tn <= CAP ? COLS : CAP / Tn;  // columns per FFT round
     static constexpr int THREADS = RC * Tn;
     static constexpr int P = COLS + 1;  // shared-memory pitch of one kz row (odd: fewer bank conflicts)
     // WZ (one round of column FFTs of at most a warp each): the forward
@@ -393,15 +398,21 @@ template <int PAD> struct IdxZ {
     __device__ __forceinline__ int operator()(int c, int e) const { return e * cols + c + (PAD ? (e >> PAD) : 0); }
 };
 
+// Blocks per SM the register budget of k_zpass_rt is set for: four with one
+// field (FP64: three, CH update 526 -> 450 us at 256^3; 512 threads: two), two
+// with three (their tiles take 105 KB and 112 KB; 512 threads: one, 210 KB).
+template <typename T, int N, int NF, int NB> struct ZRtBlocks {
+    static constexpr bool ONE = NF == 1 && NB == 1, BIG = sizeof(T) == 4 && N == 512;
+    static constexpr int value = ONE ? (BIG ? 2 : sizeof(T) == 4 ? 4 : 3) : (BIG ? 1 : 2);
+};
+
 // The tile is COLS columns (a 128-byte run of ky per kz for FP32 and FP64)
 // of all kz; the column FFTs run in rounds of RC columns, while loads and
 // the mid operation walk the tile with ky fastest (full runs per warp).
 // Tiles whose load() only copies arrays (src()) arrive by cp.async.
-// Blocks per SM: four with one field (FP64: three, CH update 526 -> 450 us at
-// 256^3), two with three (their tiles take 105 KB and
-// 112 KB; FP32 projection at 512^3 2268 -> 1990 us against no bound).
 template <typename T, int NF, int NB, int DIR, int N, int COLS, class Op, int EM = FftE<T>::value>
-__global__ void __launch_bounds__(kThreads, NF == 1 && NB == 1 ? (sizeof(T) == 4 ? 4 : 3) : 2) k_zpass_rt(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
+__global__ void __launch_bounds__(ZRtShape<T, N, COLS, EM>::CAP, ZRtBlocks<T, N, NF, NB>::value)
+    k_zpass_rt(Geom g, const tw_t<T>* __restrict__ twz, Op op) {
     using C = cplx<T>;
     constexpr bool FX = sizeof(T) == sizeof(double);  // transforms in block fixed point
     using SH = ZRtShape<T, N, COLS, EM>;

@@ -1066,12 +1066,10 @@ void launch_zrt(fipi_ctx* ctx, const char* name, int nspec, const Op& op) {
     dispatch_pow2<8, 512>(g.nz, [&](auto NC) {
         constexpr int N = decltype(NC)::value;
         constexpr int NS = NF > NB ? NF : NB;
-        // columns of 512 modes with three or more fields: half the tile (two blocks per SM)
-        constexpr int CW = (N >= 512 && NS >= 3 && COLS > 8) ? COLS / 2 : COLS;
-        using SHP = ZRtShape<T, N, CW, EM>;
+        using SHP = ZRtShape<T, N, COLS, EM>;
         const size_t smem = (size_t)NS * SHP::FSTRIDE * sizeof(cplx<T>);
-        dim3 grid(g.h, g.ny / CW);
-        auto kern = k_zpass_rt<T, NF, NB, DIR, N, CW, Op, EM>;
+        dim3 grid(g.h, g.ny / COLS);
+        auto kern = k_zpass_rt<T, NF, NB, DIR, N, COLS, Op, EM>;
         static size_t granted = 48 * 1024;
         ensure_smem(kern, smem, granted);
         kern<<<grid, SHP::BLOCK, smem, ctx->stream>>>(g, F<T>::tw(ctx, 2), op);
