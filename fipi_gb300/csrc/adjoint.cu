@@ -980,13 +980,15 @@ fipi_status fipi_trajectory_backward(fipi_ctx* ctx, const double* dc, const doub
             st = adjoint_reverse_pair(ctx, tr->K + j, tr->K + j + 1, a.seg_tape + 4 * V * (size_t)j);
             if (st != FIPI_OK) return st;
         }
-        st = check_status(ctx);
+        if (k == 0) {
+            // the context is left in the state after the trajectory's first step
+            tr->t0 = -1;  // no longer the trajectory's end
+            st = ck_load(ctx, tr->K + 1);
+            if (st != FIPI_OK) return st;
+        }
+        st = check_status(ctx);  // waits: the state and the gradients are complete at return
         if (st != FIPI_OK) return st;
     }
-    // the context is left in the state after the trajectory's first step
-    st = ck_load(ctx, tr->K + 1);
-    if (st != FIPI_OK) return st;
-    tr->t0 = -1;  // the state is no longer the trajectory's end
     return FIPI_OK;
 }
 
