@@ -16,10 +16,11 @@ def test_backward_returns_with_the_state_in_place(fipi):
     P = w.params()
     c = fipi.seed_phase(P, 3, 0.0, 0.05)
     with fipi.Simulation(P, "fp64") as s:
-        stream = torch.cuda.ExternalStream(s.stream())
         s.set_phase(c)
         s.step(1)
         first = s.get_phase()
+    with fipi.Simulation(P, "fp64") as s:
+        stream = torch.cuda.ExternalStream(s.stream())
         s.set_phase(c)
         s.trajectory_forward(2, 2)
         s.trajectory_backward(c)
