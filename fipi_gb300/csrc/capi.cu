@@ -93,6 +93,16 @@ using namespace fipi;
 // 128^3 213 -> 280; FP64 64^3 206 -> 200, 128^3 820 -> 850 (up to 2^18 nodes).
 constexpr long long kBranchMixedMaxV = 1ll << 21, kBranchSpreadMaxV = 1ll << 18;
 
+// The runtime calls of branch.hpp.
+struct CudaBranches {
+    static int stream(cudaStream_t* s) { return (int)cudaStreamCreateWithFlags(s, cudaStreamNonBlocking); }
+    static int event(cudaEvent_t* e) { return (int)cudaEventCreateWithFlags(e, cudaEventDisableTiming); }
+    static int record(cudaEvent_t e, cudaStream_t s) { return (int)cudaEventRecord(e, s); }
+    static int wait(cudaStream_t s, cudaEvent_t e) { return (int)cudaStreamWaitEvent(s, e, 0); }
+    static void drop(cudaStream_t s) { cudaStreamDestroy(s); }
+    static void drop(cudaEvent_t e) { cudaEventDestroy(e); }
+};
+
 static bool pow2_in(int n, int lo, int hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
 
 static fipi_status validate(const fipi_params* P, fipi_precision prec) {
@@ -251,9 +261,10 @@ fipi_status fipi_destroy(fipi_ctx* ctx) {
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->status_pin) cudaFreeHost(ctx->status_pin);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
-    if (ctx->side) cudaStreamDestroy(ctx->side);
-    for (cudaEvent_t ev : {ctx->fork[0], ctx->fork[1], ctx->join[0], ctx->join[1]})
-        if (ev) cudaEventDestroy(ev);
+    {
+        CudaBranches rt;
+        drop_branches(rt, ctx->side, ctx->branch);
+    }
     delete ctx;
     return FIPI_OK;
 }
@@ -512,45 +523,35 @@ void fipi::graphs_reset(fipi_ctx* ctx) {
 }
 
 
-// Runs f with the context stream replaced by the side stream, which waits for
-// the context stream's work so far (fork); the context stream waits for it in
-// join_branch.
-template <class F> static void on_branch(fipi_ctx* ctx, int k, F&& f) {
-    cudaEventRecord(ctx->fork[k], ctx->stream);
-    cudaStreamWaitEvent(ctx->side, ctx->fork[k], 0);
-    std::swap(ctx->stream, ctx->side);
-    f();
-    std::swap(ctx->stream, ctx->side);
-    cudaEventRecord(ctx->join[k], ctx->side);
-}
-static void join_branch(fipi_ctx* ctx, int k) { cudaStreamWaitEvent(ctx->stream, ctx->join[k], 0); }
-
 // One iteration of main.cpp:75-219, enqueued on the context stream.
 //
 // With `branches` the particle stages (which read c and grad c) run beside the
 // projection (fluid coupling needs the projected velocity first) and, on the
 // smallest grids, the spreading (which reads the previous step's particles and
-// writes the spread grid) beside the Cahn-Hilliard part.
-void fipi::enqueue_step(fipi_ctx* ctx, bool branches) {
+// writes the spread grid) beside the Cahn-Hilliard part.  Returns the first error
+// of a fork or join; the step is then not to be used (graph_step drops it).
+cudaError_t fipi::enqueue_step(fipi_ctx* ctx, bool branches) {
     const int t = ctx->t;
     const bool parts = ctx->pb.n > 0 && ctx->P.switch_particle;
     if (branches && parts) {
+        CudaBranches rt;
+        StepBranches<CudaBranches, cudaStream_t, cudaEvent_t> br{rt, ctx->stream, ctx->side, ctx->branch};
         const bool early = ctx->g.V <= kBranchSpreadMaxV;
-        if (early) on_branch(ctx, 0, [&] { particles_spread(ctx); });
+        if (early) br.fork(0, [&] { particles_spread(ctx); });
         fields_step_ch(ctx, t);
-        if (early) join_branch(ctx, 0);
+        if (early) br.join(0);
         else particles_spread(ctx);
         fields_step_force(ctx);
         if (ctx->couple_u) {
             fields_step_project(ctx);
             particles_step(ctx);
         } else {
-            on_branch(ctx, 1, [&] { particles_step(ctx); });
+            br.fork(1, [&] { particles_step(ctx); });
             fields_step_project(ctx);
-            join_branch(ctx, 1);
+            br.join(1);
         }
         ctx->t = t + 1;
-        return;
+        return (cudaError_t)br.err;
     }
     fields_step_ch(ctx, t);      // main.cpp:79-141
     particles_spread(ctx);       // main.cpp:169 (compute_f_r of the previous step's state)
@@ -558,6 +559,7 @@ void fipi::enqueue_step(fipi_ctx* ctx, bool branches) {
     if (!particles_step(ctx))    // main.cpp:186-219
         step_tick(ctx);
     ctx->t = t + 1;
+    return cudaSuccess;
 }
 
 extern "C" {
@@ -583,14 +585,14 @@ static fipi_status graph_step(fipi_ctx* ctx, bool* done) {
         cudaGraph_t graph = nullptr;
         if (!ctx->side && ctx->pb.n > 0 && ctx->P.switch_particle &&
             (ctx->prec == FIPI_FP64 || ctx->g.V <= kBranchMixedMaxV)) {
-            FIPI_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-            for (cudaEvent_t* ev : {&ctx->fork[0], &ctx->fork[1], &ctx->join[0], &ctx->join[1]})
-                FIPI_CUDA(ctx, cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+            CudaBranches rt;
+            if (make_branches(rt, ctx->side, ctx->branch)) cudaGetLastError();  // one chain instead
         }
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            enqueue_step(ctx, ctx->side != nullptr);
+            const cudaError_t es = enqueue_step(ctx, ctx->side != nullptr);
             e = cudaStreamEndCapture(ctx->stream, &graph);
+            if (e == cudaSuccess) e = es;
         }
         cudaGraphExec_t exec = nullptr;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/fipi.h"
+#include "branch.hpp"
 #include "fft.cuh"
 
 namespace fipi {
@@ -213,7 +214,7 @@ struct fipi_ctx {
     } graphs[2];
     bool use_graphs = true;
     cudaStream_t side = nullptr;  // second branch of the step graph (small grids)
-    cudaEvent_t fork[2] = {}, join[2] = {};
+    fipi::BranchEvents<cudaEvent_t> branch;
     int substep = 0;           // 1 after fipi_step_ch, 2 after fipi_step_stokes
     double* pin = nullptr;     // pinned host staging of the particle state, 12 n doubles
     double* pin_dev = nullptr; // the same buffer as a device pointer (mapped pinned memory)
@@ -300,8 +301,9 @@ fipi_status particles_wrap(fipi_ctx* ctx, double* p_host);
 
 // Reverse mode (adjoint.cu / particles.cu).
 // One forward step; `branches`: with the particle work on ctx->side where
-// nothing orders it behind the grid work (step graphs of small grids).
-void enqueue_step(fipi_ctx* ctx, bool branches = false);
+// nothing orders it behind the grid work (step graphs); the first error of a
+// fork or join.
+cudaError_t enqueue_step(fipi_ctx* ctx, bool branches = false);
 // Sets the device step index and the ramp factor of step t (particles.cu).
 void set_tick(fipi_ctx* ctx, int t);
 // *rmp = ramp(t + 1, 0.2 t_end).
