@@ -28,7 +28,8 @@
 //
 // Rows with an infinity or a NaN (E = 0x7ff) come out as NaN throughout.
 // Rows below 2^-959 are scaled up by 2^200 first, so subnormal inputs
-// enter with all their bits; results below 2^-1022 flush to zero.
+// enter with all their bits; results are representable up to the largest FP64
+// value and down to its subnormals (fx_unrow).
 #pragma once
 
 #include <type_traits>
@@ -138,25 +139,21 @@ __device__ __forceinline__ long long fx_from(double x, int E, int B) {
     const long long r = (long long)(m >> s);
     return hi < 0 ? -r : r;
 }
-// a 2^q, rounded to nearest (the rounding carry runs into the exponent field).
+// a 2^q, rounded to nearest (the rounding carry runs into the exponent field),
+// for -1022 <= q <= 960, where every result but zero is a normal number.
 __device__ __forceinline__ double fx_to(long long a, int q) {
     const int sg = fx_hi(a) & 0x80000000;
     const unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
     const int z = __clzll((long long)u);  // >= 1: |a| < 2^63
     const unsigned long long r = ((u << (z - 1)) + 0x200ull) >> 10;  // leading one at bit 52
     const int e = q + 1085 - z;  // exponent field less one (1023 + 63)
-    if (u == 0 || (unsigned)e >= 2045u)  // zero, or outside the normal range
-        return u == 0 || e < 0 ? 0.0 : __hiloint2double(sg | 0x7ff00000, 0);
-    return __hiloint2double(((int)(r >> 32) + (e << 20)) | sg, (int)(unsigned)r);
+    return u == 0 ? 0.0 : __hiloint2double(((int)(r >> 32) + (e << 20)) | sg, (int)(unsigned)r);
 }
 // The same by the FP64 pipe's conversion instruction and an exponent addition:
 // one FP64 instruction instead of a dozen integer ones.
 __device__ __forceinline__ double fx_to_cvt(long long a, int q) {
     const double d = __ll2double_rn(a);
-    const int h = __double2hiint(d), e = ((h >> 20) & 0x7ff) + q;
-    if (a == 0 || (unsigned)(e - 1) >= 2046u)
-        return a == 0 || e < 1 ? 0.0 : __hiloint2double((h & 0x80000000) | 0x7ff00000, 0);
-    return __hiloint2double(h + (q << 20), __double2loint(d));
+    return a == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (q << 20), __double2loint(d));
 }
 // One component on either pipe: 1099 G conversions/s against 844 (integer)
 // and 593 (FP64 pipe), measured alone.
@@ -199,8 +196,19 @@ template <int K, int BITS, int L1> __device__ __forceinline__ FxExp fx_row(doubl
 }
 // Integers of such a row back to FP64, times 2^shift.
 template <int K> __device__ __forceinline__ void fx_unrow(const longlong2* o, FxExp x, int shift, double2* v) {
+    // rows whose values may leave the normal range: converted inside it, then
+    // scaled by a power of two, which rounds subnormals and overflows as FP64 does
+    const int q = x.q + shift, adj = q < -1022 ? 400 : q > 960 ? -200 : 0;
 #pragma unroll
-    for (int i = 0; i < K; ++i) v[i] = fx_to(o[i], x.q + shift);
+    for (int i = 0; i < K; ++i) v[i] = fx_to(o[i], q + adj);
+    if (adj != 0) {
+        const double f = adj > 0 ? 0x1p-400 : 0x1p200;
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            v[i].x *= f;
+            v[i].y *= f;
+        }
+    }
     if (x.E == 0x7ff) {
 #pragma unroll
         for (int i = 0; i < K; ++i) v[i].x = v[i].y = __hiloint2double(0x7ff80000, 0);
