@@ -1,0 +1,39 @@
+// FP64 quotients for GB300, whose FP64 pipe issues at 1/64 of the FP32 rate: a
+// division is some ten FP64 instructions.  Source of its own so that a host
+// program can compile it and compare with the division.
+#pragma once
+
+namespace fipi {
+
+// 1/x as an unevaluated sum hi + lo, to about 104 bits.
+struct Recip {
+    double hi, lo;
+};
+// From an FP32 estimate r (converted both ways on the bits; a conversion or a
+// division runs on the FP64 pipe) one third-order step r (1 + e + e^2),
+// e = 1 - x r, |e| < 2^-20, gives hi; the remainder of hi gives lo: five FP64
+// instructions.  x outside (2^-126, 2^126), negative or NaN: the division.
+__device__ __forceinline__ Recip recip(double x) {
+    Recip o;
+    const int h = __double2hiint(x);
+    if ((unsigned)(h - ((1023 - 126) << 20)) >= (252u << 20)) {
+        o.hi = 1.0 / x;
+        o.lo = fma(-x, o.hi, 1.0) * o.hi;
+        if (!(fabs(o.lo) < fabs(o.hi))) o.lo = 0.0;  // 0, infinity, NaN
+        return o;
+    }
+    const float r0 = __fdividef(1.f, __int_as_float(((h - (896 << 20)) << 3) | (int)((unsigned)__double2loint(x) >> 29)));
+    const int b = __float_as_int(r0);
+    const double r = __hiloint2double((b >> 3) + (896 << 20), b << 29);
+    const double e = fma(-x, r, 1.0);
+    o.hi = fma(r, fma(e, e, e), r);
+    o.lo = fma(-x, o.hi, 1.0) * o.hi;
+    return o;
+}
+// a / x, two FP64 instructions: a lo carries a relative error of 2^-53 on at
+// most 2^-52 of the quotient, and the sum is rounded once, so the result is
+// the division's unless the quotient lies within 2^-103 of the middle of two
+// values.  (Quotients below 2^-960 keep one unit; an infinite a may give NaN.)
+__device__ __forceinline__ double over(double a, Recip r) { return fma(a, r.hi, a * r.lo); }
+
+}  // namespace fipi

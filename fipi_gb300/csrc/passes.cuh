@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "ctx.hpp"
+#include "fp64.cuh"
 
 namespace fipi {
 

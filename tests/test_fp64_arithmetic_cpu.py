@@ -1,0 +1,68 @@
+"""The FP64 quotients of csrc/fp64.cuh, compiled for the host, against the
+division they stand for."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+REPO = Path(__file__).resolve().parent.parent
+
+# CUDA's names for the host.  The FP32 reciprocal estimate is off by up to the
+# two units its documentation allows.
+HOST = r"""
+#include <cmath>
+#include <cstdint>
+#include <cstdio>
+#include <cstring>
+#include <random>
+#define __device__
+#define __forceinline__ inline
+using std::fabs; using std::fma;
+static std::mt19937_64 rng(7);
+template <class A, class B> static A bits(B b) { A a; std::memcpy(&a, &b, sizeof a); return a; }
+static int __double2hiint(double x) { return (int)(bits<uint64_t>(x) >> 32); }
+static int __double2loint(double x) { return (int)(uint32_t)bits<uint64_t>(x); }
+static double __hiloint2double(int h, int l) { return bits<double>(((uint64_t)(uint32_t)h << 32) | (uint32_t)l); }
+static long long __double_as_longlong(double x) { return bits<long long>(x); }
+static float __int_as_float(int i) { return bits<float>(i); }
+static int __float_as_int(float f) { return bits<int>(f); }
+static float __fdividef(float a, float b) { return __int_as_float(__float_as_int(a / b) + (int)(rng() % 5) - 2); }
+#include "fp64.cuh"
+using namespace fipi;
+// random mantissa and sign, exponent in [lo, hi)
+static double draw(int lo, int hi) {
+    const uint64_t m = rng();
+    return std::ldexp(1.0 + (double)(m >> 12) * 0x1p-52, lo + (int)(rng() % (uint64_t)(hi - lo))) * (m & 1 ? -1 : 1);
+}
+"""
+
+OVER = r"""
+int main() {
+    long bad = 0;
+    const int ranges[][4] = {{-60, 20, 1, 40}, {-300, 300, -125, 126}, {-400, 400, -200, 300}};
+    for (auto& r : ranges)
+        for (long i = 0; i < 4000000; ++i) {
+            const double a = draw(r[0], r[1]), x = fabs(draw(r[2], r[3]));
+            bad += over(a, recip(x)) != a / x;
+        }
+    for (double a : {0.0, 1.0, -3.5})
+        for (double x : {3.0, 0x1p-126, 0x1p126, 0x1p-1022, (double)INFINITY}) bad += over(a, recip(x)) != a / x;
+    bad += over(1.0, recip(0.0)) != INFINITY || !std::isnan(over(0.0, recip(0.0))) || !std::isnan(over(1.0, recip(NAN)));
+    std::printf("%ld\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def _run(tmp_path, body):
+    src, exe = tmp_path / "h.cpp", tmp_path / "h"
+    src.write_text(HOST + body)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", str(REPO / "fipi_gb300/csrc"), str(src),
+                    "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("body", [OVER], ids=["over"])
+def test_quotients_are_the_divisions(tmp_path, body):
+    _run(tmp_path, body)
