@@ -531,7 +531,7 @@ void adjoint_fields(fipi_ctx* ctx, bool first) {
     OpR2CN<D, 3> o1{{a.la_u, a.la_u + V, a.la_u + 2 * V}, {S[0], S[1], S[2]}, g.nx, g.ny};
     launch_x<D, 0, 3, false>(ctx, "adjoint: X forward u", 3, NoAcc<OpR2CN<D, 3>>{o1});
     launch_y<D>(ctx, 3, Sv, Sv, -1);
-    ZOpProj<D> zp{{S[0], S[1], S[2]}, {S[0], S[1], S[2]}, kt, k.mu, 1.0 / ctx->P.mu, g.m, g.ny / 2, g.nz / 2};
+    ZOpProj<D> zp{{S[0], S[1], S[2]}, {S[0], S[1], S[2]}, kt, k.mu, g.m, g.ny / 2, g.nz / 2};
     launch_z<D, 3, -1>(ctx, "adjoint: Z forward + projection", 6, zp);
     // lamF real, Stokes pointwise adjoint, 5 forward transforms
     ZOpStore<D, 3> zi{{S[0], S[1], S[2]}, {S[0], S[1], S[2]}, 0};

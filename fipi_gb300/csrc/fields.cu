@@ -958,7 +958,7 @@ template <typename T> static void step_project_t(fipi_ctx* ctx) {
     const KTabs<T> kt = F<T>::ktabs(ctx);
     void* s3[3] = {b.S[0], b.S[1], b.S[2]};
     launch_y<T>(ctx, 3, s3, s3, -1);
-    ZOpProj<T> zp{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, {nullptr, nullptr, nullptr}, kt, k.mu, T(1.0 / ctx->P.mu), g.m,
+    ZOpProj<T> zp{{F<T>::S(ctx, 0), F<T>::S(ctx, 1), F<T>::S(ctx, 2)}, {nullptr, nullptr, nullptr}, kt, k.mu, g.m,
                   g.ny / 2, g.nz / 2};
     ZOpProjRt<T> zpr{zp, {F<T>::sp(b.upre[0]), F<T>::sp(b.upre[1]), F<T>::sp(b.upre[2])}};
     launch_zrt<T, 3, 3, -1, 16 / (sizeof(T) / 4), true>(ctx, "Z forward + projection + inverse", 6, zpr);

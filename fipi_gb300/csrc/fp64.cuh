@@ -36,4 +36,9 @@ __device__ __forceinline__ Recip recip(double x) {
 // values.  (Quotients below 2^-960 keep one unit; an infinite a may give NaN.)
 __device__ __forceinline__ double over(double a, Recip r) { return fma(a, r.hi, a * r.lo); }
 
+// The projection of one mode (main.cpp:177-178), f - k (k.f)/k^2 over mu k^2, a
+// component at a time: s = (k.f)/k^2, r = 1/(mu k^2).  Three roundings, a fused
+// multiply-add among them, where the reference's order has four.
+__device__ __forceinline__ double projected(double f, double k, double s, Recip r) { return over(fma(-k, s, f), r); }
+
 }  // namespace fipi

@@ -65,21 +65,6 @@ template <typename T> struct KTabs {
     }
 };
 
-// 1/x in FP64 from an FP32 estimate (converted both ways on the bits; a
-// conversion or a division runs on the FP64 pipe, which issues at 1/64 of the
-// FP32 rate) and one third-order step r (1 + e + e^2), e = 1 - x r, |e| <
-// 2^-20: three FP64 instructions, within 1.5 units in the last place.  x
-// outside (2^-126, 2^126), negative or NaN: the division.
-__device__ __forceinline__ double fast_inv(double x) {
-    const int h = __double2hiint(x);
-    if ((unsigned)(h - ((1023 - 126) << 20)) >= (252u << 20)) return 1.0 / x;
-    const float r0 = __fdividef(1.f, __int_as_float(((h - (896 << 20)) << 3) | (int)((unsigned)__double2loint(x) >> 29)));
-    const int b = __float_as_int(r0);
-    const double r = __hiloint2double((b >> 3) + (896 << 20), b << 29);
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 // ------------------------------------------------------------ block reduce
 __device__ __forceinline__ double block_sum(double v) {
     __shared__ double red[32];
@@ -805,14 +790,14 @@ template <typename T> struct ZOpProj {
     C* out[3];
     __device__ const C* src(int f) const { return in[f]; }
     KTabs<T> kt;
-    T mu, inv_mu;
+    T mu;
     int m, ny2, nz2;
     __device__ void load(int, int, int, size_t gi, C* v) const {
         v[0] = in[0][gi];
         v[1] = in[1][gi];
         v[2] = in[2][gi];
     }
-    __device__ void project(const T* kv, T k2, T mk2, const C* F, C* u) const {
+    __device__ static void project(const T* kv, T k2, T mk2, const C* F, C* u) {
         T dre = T(0), dim = T(0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -828,14 +813,14 @@ template <typename T> struct ZOpProj {
                 u[d] = mkc<C>((F[d].x - qre) * r2, (F[d].y - qim) * r2);
             }
         } else {
-            // FP64: (F - k (k.F)/k^2) / (mu k^2) with one reciprocal instead of
-            // twelve divisions (a division is some ten FP64 instructions;
-            // 2551 -> 1131 us at 256^3 with the warp-owned columns)
-            const T r1 = fast_inv(k2), r2 = r1 * inv_mu;
-            dre *= r1;
-            dim *= r1;
+            // FP64: two reciprocals with their remainders instead of twelve
+            // divisions (fp64.cuh; 1205 us a round trip at 256^3, where
+            // rounded reciprocals and their larger errors took 1096)
+            const Recip r1 = recip(k2), r2 = recip(mk2);
+            dre = over(dre, r1);
+            dim = over(dim, r1);
 #pragma unroll
-            for (int d = 0; d < 3; ++d) u[d] = mkc<C>(fma(-kv[d], dre, F[d].x) * r2, fma(-kv[d], dim, F[d].y) * r2);
+            for (int d = 0; d < 3; ++d) u[d] = mkc<C>(projected(F[d].x, kv[d], dre, r2), projected(F[d].y, kv[d], dim, r2));
         }
     }
     __device__ void store(int ix, int iy, int iz, size_t gi, const C* F) const {
