@@ -5,6 +5,19 @@
 
 namespace fipi {
 
+// a / b with r = 1/b rounded to nearest at hand: the quotient estimate corrected
+// by its exact remainder is the correctly rounded quotient (P. Markstein, IBM J.
+// Res. Dev. 34, 1990), so the results are those of the division, in three
+// FP64 instructions instead of about ten.  Infinite, NaN and extreme values
+// take the division: quotients outside 2^-512 to 2^512, and numerators below 2^-959,
+// whose remainder would lose bits below the subnormals.  |b| < 2^1000.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    const double q = a * r;
+    const int e = (__double2hiint(q) >> 20) & 0x7ff, ea = (__double2hiint(a) >> 20) & 0x7ff;
+    if ((unsigned)(e - 511) > 1024u || ea < 64) return (__double_as_longlong(a) << 1) == 0 ? q : a / b;
+    return fma(fma(-q, b, a), r, q);
+}
+
 // 1/x as an unevaluated sum hi + lo, to about 104 bits.
 struct Recip {
     double hi, lo;

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "ctx.hpp"
+#include "fp64.cuh"
 #include "fixed_point.cuh"
 
 namespace fipi {
@@ -217,19 +218,6 @@ static int bits_for(long long maxval) {
     int b = 1;
     while ((1ll << b) <= maxval) ++b;
     return b;
-}
-
-// a / b with r = 1/b rounded to nearest at hand: the quotient estimate corrected
-// by its exact remainder is the correctly rounded quotient (P. Markstein, IBM J.
-// Res. Dev. 34, 1990), so the results are those of the division, in three
-// FP64 instructions instead of about ten.  Infinite, NaN and extreme values
-// (where the remainder would not be exact) take the division; b is finite and
-// not zero.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-    const double q = a * r;
-    const int e = (__double2hiint(q) >> 20) & 0x7ff;  // between 2^-512 and 2^512: nothing under- or overflows
-    if ((unsigned)(e - 511) > 1024u) return (__double_as_longlong(a) << 1) == 0 ? q : a / b;
-    return fma(fma(-q, b, a), r, q);
 }
 
 // ------------------------------------------------------------ cell list

@@ -3,6 +3,8 @@ division they stand for."""
 import subprocess
 from pathlib import Path
 
+import pytest
+
 REPO = Path(__file__).resolve().parent.parent
 
 # CUDA's names for the host.  The FP32 reciprocal estimate is off by up to the
@@ -46,6 +48,25 @@ int main() {
     for (double a : {0.0, 1.0, -3.5})
         for (double x : {3.0, 0x1p-126, 0x1p126, 0x1p-1022, (double)INFINITY}) bad += over(a, recip(x)) != a / x;
     bad += over(1.0, recip(0.0)) != INFINITY || !std::isnan(over(0.0, recip(0.0))) || !std::isnan(over(1.0, recip(NAN)));
+    std::printf("%ld\n", bad);
+    return bad != 0;
+}
+"""
+
+DIV_BY = r"""
+int main() {
+    long bad = 0;
+    const int ranges[][4] = {{-60, 60, -40, 40}, {-1074, 1000, -1000, 999}, {-1074, -900, -1000, -400}};
+    for (auto& r : ranges)
+        for (long i = 0; i < 4000000; ++i) {
+            const double a = draw(r[0], r[1]), b = draw(r[2], r[3]);
+            bad += bits<uint64_t>(div_by(a, b, 1.0 / b)) != bits<uint64_t>(a / b);
+        }
+    for (double a : {0.0, -0.0, 1.0, (double)INFINITY, (double)NAN})
+        for (double b : {3.0, -3.0, 0.0, (double)INFINITY, (double)NAN}) {
+            const double x = div_by(a, b, 1.0 / b), y = a / b;
+            bad += std::isnan(y) ? !std::isnan(x) : x != y || std::signbit(x) != std::signbit(y);
+        }
     std::printf("%ld\n", bad);
     return bad != 0;
 }
@@ -98,8 +119,9 @@ def _run(tmp_path, body):
     return r.stdout
 
 
-def test_quotients_are_the_divisions(tmp_path):
-    _run(tmp_path, OVER)
+@pytest.mark.parametrize("body", [OVER, DIV_BY], ids=["over", "div_by"])
+def test_quotients_are_the_divisions(tmp_path, body):
+    _run(tmp_path, body)
 
 
 def test_projection_is_as_accurate_as_the_reference(tmp_path):
