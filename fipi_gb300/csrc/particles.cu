@@ -60,7 +60,7 @@ struct PC {
     double drag;       // 6 pi mu: the Stokes drag is drag * r
     double img[3];     // d_cell (n_cell - 2): the minimum-image threshold
     double inv_req2;    // 1/r_eq^2
-    float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
+    float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_gap[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
 };
 
 static PC make_pc(const fipi_ctx* ctx) {
@@ -97,6 +97,7 @@ static PC make_pc(const fipi_ctx* ctx) {
         c.inv_dc[a] = 1.0 / c.dc[a];
         c.mdc[a] = c.margin / c.dc[a];
         c.f_dc[a] = (float)c.dc[a];
+        c.f_gap[a] = (float)(c.dc[a] * c.nc[a] - c.L[a]);
         c.img[a] = c.dc[a] * (c.nc[a] - 2);
     }
     c.drag = 6.0 * c.pi * c.mu;
@@ -106,8 +107,8 @@ static PC make_pc(const fipi_ctx* ctx) {
     c.f_req2 = c.f_req * c.f_req;
     c.inv_req2 = 1.0 / (c.r_eq * c.r_eq);
     // FP32 selection radius: a separation formed from cell-relative FP32
-    // coordinates of up to 2 d_cell is off by less than 16 * 2^-24 d_cell per
-    // axis (two conversions, the offset and its product, two subtractions)
+    // coordinates of up to 3 d_cell is off by less than 16 * 2^-24 d_cell per
+    // axis (two conversions, the offset and its terms, two subtractions)
     {
         const double dcm = std::max(c.dc[0], std::max(c.dc[1], c.dc[2]));
         const double rs = c.r_eq + 32.0 * dcm / 16777216.0;
@@ -650,12 +651,23 @@ __global__ void k_sorted_pos(PC pc, const double* __restrict__ p, const unsigned
     sorted_pos(pc, p, (int)ids[s], key % pc.nc[0], (key / pc.nc[0]) % pc.nc[1], key / (pc.nc[0] * pc.nc[1]), s, spos);
 }
 
+// Origin of the neighbour cell at c + dc (dc = -1, 0, 1) of the periodic cell
+// grid relative to cell c's, in the image the reference's rule gives: dc
+// cells, and through the periodic wrap L instead of n_cell d_cell.  The two
+// differ (f_gap) where margin != 0, and where L / r_c rounds up to a whole
+// number: fmod(L, r_c) is then nearly r_c and the cells reach one r_c beyond L
+// (cluster.cpp:26-32).  f_gap is 0 to rounding otherwise and changes no bit.
+__device__ __forceinline__ float cell_offset(const PC& pc, int a, int c, int dc) {
+    const float o = (float)dc * pc.f_dc[a];
+    return c + dc < 0 ? o + pc.f_gap[a] : c + dc >= pc.nc[a] ? o - pc.f_gap[a] : o;
+}
+
 // Mixed-form contact forces when every axis has at least 4 cells.  Then
 // the reference's minimum-image rule (shift d by L when |d| exceeds
 // d_cell (n_cell - 2), cluster.cpp:225-232) shifts exactly the pairs whose
 // neighbour cell was reached through the periodic wrap, so d can be formed
 // from cell-relative FP32 coordinates plus the neighbour cell's offset
-// (di, dj, dk) d_cell, with no per-pair test.  The force on the home
+// (cell_offset), with no per-pair test.  The force on the home
 // particle from a pair is (d/|d|) s with d = p_i - p_j for either id
 // order (exactly the reference's sign rule), summed in the reference's
 // cell order.
@@ -708,7 +720,7 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
     float rmp = 0.f;
     if (lane == 0) rmp = (float)*rmp_p;
     rmp = __shfl_sync(0xffffffffu, rmp, 0);
-    const float dcx = pc.f_dc[0], dcy = pc.f_dc[1], dcz = pc.f_dc[2];
+    const float oy = cell_offset(pc, 1, cj, dj), oz = cell_offset(pc, 2, ck, dk);
     bool mark_ok = false;
     if (f_pi != nullptr) {
         const int m = *it_mark;
@@ -733,9 +745,8 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
         float ax = 0.f, ay = 0.f, az = 0.f, tau = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const int di = c - 1;
             // home particle relative to the neighbour cell's origin (home frame)
-            const float hx = h.x - di * dcx, hy = h.y - dj * dcy, hz = h.z - dk * dcz;
+            const float hx = h.x - cell_offset(pc, 0, ci, c - 1), hy = h.y - oy, hz = h.z - oz;
             for (int q0 = qb[c]; q0 < qe[c]; q0 += 32) {
                 if (q0 != held[c]) {  // a cell of more than 32 particles: stage its next chunk
                     __syncwarp();
@@ -808,8 +819,8 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
 //
 // The block stages the candidates of the 27 neighbour cells in shared memory
 // in the reference's cell order, as FP32 positions in the home cell's frame
-// (cell-relative coordinates plus the neighbour cell's offset (di, dj, dk)
-// d_cell).  About one candidate in twelve lies within r_eq (4/3 pi r_eq^3
+// (cell-relative coordinates plus the neighbour cell's offset, cell_offset).
+// About one candidate in twelve lies within r_eq (4/3 pi r_eq^3
 // against 27 cells), so these separations only select: candidates within
 // r_eq plus their rounding bound (f_req2_sel) are queued by ballot, and every
 // 32 of them are evaluated with all lanes busy, from FP64 separations
@@ -819,7 +830,7 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
 // the rule for every pair that
 // can interact: with at least 4 cells per axis the rule shifts exactly the
 // pairs reached through the periodic wrap, and with 3 it differs only for
-// pairs further apart than d_cell; f_pp_path asks for r_eq <= d_cell
+// pairs further apart than L - 2 d_cell; f_pp_path asks for r_eq to be below
 // there.  Lane sums meet in a fixed shuffle order:
 // deterministic.
 constexpr int kFppWarps = 4;
@@ -829,6 +840,7 @@ struct FppShared {
     float4 cand[kFppStage];  // x, y, z in the home cell's frame, id
     int queue[kFppWarps][64];
     int beg[27], pre[28];  // start and exclusive count prefix of the neighbour cells
+    float ofs[27][3];      // cell_offset of each
 };
 
 // Starts and prefix counts of the 27 neighbour cells (first warp).
@@ -839,6 +851,9 @@ __device__ __forceinline__ void fpp_cells(const PC& pc, int cell, const int* __r
     int beg = 0, cnt = 0;
     if (lane < 27) {
         int i = ci + lane % 3 - 1, j = cj + (lane / 3) % 3 - 1, k = ck + lane / 9 - 1;
+        sh.ofs[lane][0] = cell_offset(pc, 0, ci, i - ci);
+        sh.ofs[lane][1] = cell_offset(pc, 1, cj, j - cj);
+        sh.ofs[lane][2] = cell_offset(pc, 2, ck, k - ck);
         i += i < 0 ? pc.nc[0] : i >= pc.nc[0] ? -pc.nc[0] : 0;
         j += j < 0 ? pc.nc[1] : j >= pc.nc[1] ? -pc.nc[1] : 0;
         k += k < 0 ? pc.nc[2] : k >= pc.nc[2] ? -pc.nc[2] : 0;
@@ -871,9 +886,9 @@ __device__ __forceinline__ void fpp_stage(const PC& pc, const float4* __restrict
             for (int step = 16; step > 0; step >>= 1)
                 if (c + step < 27 && sh.pre[c + step] <= g) c += step;
             v = spos[sh.beg[c] + (g - sh.pre[c])];
-            v.x += (float)(c % 3 - 1) * pc.f_dc[0];
-            v.y += (float)((c / 3) % 3 - 1) * pc.f_dc[1];
-            v.z += (float)(c / 9 - 1) * pc.f_dc[2];
+            v.x += sh.ofs[c][0];
+            v.y += sh.ofs[c][1];
+            v.z += sh.ofs[c][2];
         }
         sh.cand[q] = v;
     }
@@ -1800,7 +1815,7 @@ static void it_mark_launch(fipi_ctx* ctx, const double* p) {
 // the mixed form with 3 cells on an axis (where its separations always came
 // from FP64 differences): k_f_pp_warp wherever its cell offsets give the
 // minimum image (see there); otherwise (margin != 0, or 3 cells on an axis and
-// r_eq > d_cell) k_f_pp, one warp per home cell in the reference's pair order.
+// r_eq > L - 2 d_cell, which is d_cell unless the cells reach beyond L) k_f_pp, one warp per home cell in the reference's pair order.
 // Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp 110;
 // 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 21; mixed, 20,000
 // particles, k_f_pp_fast 27.
@@ -1809,8 +1824,11 @@ static FppPath f_pp_path(const fipi_ctx* ctx, bool fp32) {
     const ParticleBufs& b = ctx->pb;
     if (fp32 && b.ncell[0] >= 4 && b.ncell[1] >= 4 && b.ncell[2] >= 4) return FppPath::fast;
     if (ctx->P.margin != 0.0) return FppPath::cell;
-    for (int a = 0; a < 3; ++a)
-        if (b.ncell[a] < 3 || (b.ncell[a] == 3 && ctx->P.r_eq > b.dcell[a])) return FppPath::cell;
+    const double L[3] = {ctx->P.lx, ctx->P.ly, ctx->P.lz};
+    for (int a = 0; a < 3; ++a) {
+        const double least = std::min(b.dcell[a], L[a] - 2.0 * b.dcell[a] * (1.0 - 1e-15));
+        if (b.ncell[a] < 3 || (b.ncell[a] == 3 && ctx->P.r_eq > least)) return FppPath::cell;
+    }
     return FppPath::warp;
 }
 
