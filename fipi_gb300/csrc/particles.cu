@@ -998,7 +998,10 @@ __device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict
 }
 
 // TA: the arithmetic the forces are formed and summed in (k_f_pp's): double in
-// the FP64 form; float in the mixed form, from the FP64 separations and added
+// the FP64 form, each pair's force being the reference's bit for bit (a square
+// root, a reciprocal and products in its order: 173 us at 256^3 where a
+// Halley step for r_eq/|d| and fused products, with 1.45 times the
+// rounding error, took 104); float in the mixed form, from the FP64 separations and added
 // one after the other in the reference's pair order, so that the mixed form's
 // forces are k_f_pp<float>'s bit for bit.
 template <typename TA>
@@ -1019,11 +1022,11 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const doubl
         const int i = __float_as_int(h.w);
         const bool tau_on = mark && any_force(f_pi, n, i);
         const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
-        const double rmp = *rmp_p, str = rmp * pc.k_n;
+        const double rmp = *rmp_p;
         TA ax = TA(0), ay = TA(0), az = TA(0);
         double tau = 0.0;
         walk([&](int j) {
-            double d[3] = {0.0, 0.0, 0.0}, d2 = 0.0;
+            double d[3] = {0.0, 0.0, 0.0};
             if (j >= 0) {
                 d[0] = min_image(xi - p[j], pc.img[0], pc.L[0]);
                 d[1] = min_image(yi - p[n + j], pc.img[1], pc.L[1]);
@@ -1049,17 +1052,18 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const doubl
                     az += __shfl_sync(0xffffffffu, fz, l);
                 }
             } else {
+                // the reference's terms, rounding by rounding (cluster.cpp:240-255)
                 if (j < 0) return;
-                d2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
-                // (r_eq - |d|) ramp k_n d / |d|  =  (r_eq/|d| - 1) ramp k_n d
-                const double y = inv_distance(d2 * pc.inv_req2);
-                const long long yb = __double_as_longlong(y);
-                if (yb <= 0x3ff0000000000000ll || yb > 0x7ff0000000000000ll) return;  // !(y > 1), on the bits
-                const double sc = fma(y, str, -str);
-                ax = fma(d[0], sc, ax);
-                ay = fma(d[1], sc, ay);
-                az = fma(d[2], sc, az);
-                if (tau_on && i < j) tau = fma(0.5 * sc, d2, tau);
+                const double dn = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+                // dn < r_eq on the bits (false for NaN)
+                if (__double_as_longlong(dn) >= __double_as_longlong(pc.r_eq)) return;
+                const double sc = (pc.r_eq - dn) * rmp * pc.k_n;
+                const Recip ir = recip(dn);
+                const double fx = over(d[0], ir) * sc, fy = over(d[1], ir) * sc, fz = over(d[2], ir) * sc;
+                ax += fx;
+                ay += fy;
+                az += fz;
+                if (tau_on && i < j) tau += fx * 0.5 * d[0] + fy * 0.5 * d[1] + fz * 0.5 * d[2];
             }
         });
         if constexpr (sizeof(TA) == sizeof(float)) {  // every lane holds the sums
@@ -1816,9 +1820,9 @@ static void it_mark_launch(fipi_ctx* ctx, const double* p) {
 // from FP64 differences): k_f_pp_warp wherever its cell offsets give the
 // minimum image (see there); otherwise (margin != 0, or 3 cells on an axis and
 // r_eq > L - 2 d_cell, which is d_cell unless the cells reach beyond L) k_f_pp, one warp per home cell in the reference's pair order.
-// Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp 110;
-// 256 particles in 3^3 cells, FP64 958 -> 16, mixed 518 -> 21; mixed, 20,000
-// particles, k_f_pp_fast 27.
+// Times: FP64, 20,000 particles at 256^3, k_f_pp 2391 us, k_f_pp_warp 173;
+// 256 particles in 3^3 cells, FP64 958 -> 20, mixed 518 -> 21; mixed, 20,000
+// particles, k_f_pp_fast 28.
 enum class FppPath { cell, warp, fast };
 static FppPath f_pp_path(const fipi_ctx* ctx, bool fp32) {
     const ParticleBufs& b = ctx->pb;
