@@ -184,17 +184,11 @@ template <typename T> struct OpForce {
         // buoyancy ((1+c)/2 rho1 + (1-c)/2 rho2) g, g = (0, 0, gravity); with
         // gravity = 0 it adds exactly zero and c is not read
         T b0 = T(0), b1 = T(0);
-        if (sizeof(T) == sizeof(double) && gravity != T(0)) {
-            // FP64: gravity (rho1 + rho2)/2 + c gravity (rho1 - rho2)/2, one
-            // instruction a point (gravity is applied here)
+        if (gravity != T(0)) {
             const C cc = r.get(0, n);
-            const T w0 = gravity * (rho1 + rho2) * T(0.5), w1 = gravity * (rho1 - rho2) * T(0.5);
-            b0 = cc.x * w1 + w0;
-            b1 = cc.y * w1 + w0;
-        } else if (gravity != T(0)) {
-            const C cc = r.get(0, n);
-            b0 = ((cc.x + T(1)) / T(2)) * rho1 + ((cc.x * T(-1) + T(1)) / T(2)) * rho2;
-            b1 = ((cc.y + T(1)) / T(2)) * rho1 + ((cc.y * T(-1) + T(1)) / T(2)) * rho2;
+            const T h1 = rho1 * T(0.5), h2 = rho2 * T(0.5);
+            b0 = mean_density(cc.x, h1, h2);
+            b1 = mean_density(cc.y, h1, h2);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -206,10 +200,7 @@ template <typename T> struct OpForce {
                 f0 += sp.x;
                 f1 += sp.y;
             }
-            if (d == 2 && sizeof(T) == sizeof(double)) {
-                f0 += b0;
-                f1 += b1;
-            } else if (d == 2 && gravity != T(0)) {
+            if (d == 2 && gravity != T(0)) {
                 f0 += b0 * gravity;
                 f1 += b1 * gravity;
             }

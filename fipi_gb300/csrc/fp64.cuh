@@ -54,4 +54,12 @@ __device__ __forceinline__ double over(double a, Recip r) { return fma(a, r.hi, 
 // multiply-add among them, where the reference's order has four.
 __device__ __forceinline__ double projected(double f, double k, double s, Recip r) { return over(fma(-k, s, f), r); }
 
+// Density at phase c, (1 + c)/2 rho1 + (1 - c)/2 rho2 (main.cpp:149-172), from the
+// halved densities, which round as the reference's order does (halving is
+// exact) in four FP64 instructions a point instead of six.  (c times half
+// the difference plus half the sum, one instruction, has errors up to 1.5 times as large.)
+template <typename T> __device__ __forceinline__ T mean_density(T c, T half1, T half2) {
+    return (c + T(1)) * half1 + (T(1) - c) * half2;
+}
+
 }  // namespace fipi

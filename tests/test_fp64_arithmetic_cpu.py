@@ -126,3 +126,25 @@ def test_quotients_are_the_divisions(tmp_path, body):
 
 def test_projection_is_as_accurate_as_the_reference(tmp_path):
     _run(tmp_path, PROJECT)
+
+
+# the buoyancy's density: the reference's expression bit for bit
+DENSITY = r"""
+int main() {
+    long bad = 0;
+    const double rho[][2] = {{1e-3, 1e-3}, {1e-3, 5e-2}, {1.0, 1e-3}, {2.0, 1.0}, {0.7, 0.3}, {1e3, 1.2}, {1.0, 0.0}};
+    for (auto& r : rho)
+        for (int i = 0; i < 1000000; ++i) {
+            const double c = i % 2 ? 1.1 * ((double)(rng() >> 11) * 0x1p-52 - 1.0) : draw(-60, 2);
+            bad += mean_density(c, r[0] * 0.5, r[1] * 0.5) != ((c + 1.0) / 2.0) * r[0] + ((c * -1.0 + 1.0) / 2.0) * r[1];
+            const float f = (float)c, r0 = (float)r[0], r1 = (float)r[1];
+            bad += mean_density(f, r0 * 0.5f, r1 * 0.5f) != ((f + 1.f) / 2.f) * r0 + ((f * -1.f + 1.f) / 2.f) * r1;
+        }
+    std::printf("%ld\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def test_density_is_the_references(tmp_path):
+    _run(tmp_path, DENSITY)
