@@ -62,4 +62,24 @@ template <typename T> __device__ __forceinline__ T mean_density(T c, T half1, T 
     return (c + T(1)) * half1 + (T(1) - c) * half2;
 }
 
+// Terms of one contact pair at distance |d| < r_eq in the adjoint of the contact
+// forces, F(d) = (r_eq - |d|) ramp k_n d / |d|: dF^T dl into lam, F . li / k_n into kn.
+// Quotients and products are the ones of
+//   a = r_eq / |d| - 1,  b = r_eq / |d|^3 (d . dl),  lam += ramp k_n (a dl - b d),
+//   kn += (r_eq - |d|) ramp / |d| (d . li).
+// (To be compiled without contraction.)
+__device__ __forceinline__ void pair_adjoint(const double d[3], double r_eq, double rmp, double k_n,
+                                             const double dl[3], const double li[3], double lam[3], double& kn) {
+    const double dn = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    // 0 < dn < r_eq on the bits (false for NaN)
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(dn);
+    if (bits == 0ull || bits >= (unsigned long long)__double_as_longlong(r_eq)) return;
+    const double sc = rmp * k_n;
+    const Recip r1 = recip(dn), r3 = recip(dn * dn * dn);
+    const double a = over(r_eq, r1) - 1.0;
+    const double b = over(r_eq, r3) * (d[0] * dl[0] + d[1] * dl[1] + d[2] * dl[2]);
+    for (int e = 0; e < 3; ++e) lam[e] += sc * (a * dl[e] - b * d[e]);
+    kn += over((r_eq - dn) * rmp, r1) * (d[0] * li[0] + d[1] * li[1] + d[2] * li[2]);
+}
+
 }  // namespace fipi

@@ -59,7 +59,6 @@ struct PC {
     double mdc[3];     // margin/d_cell
     double drag;       // 6 pi mu: the Stokes drag is drag * r
     double img[3];     // d_cell (n_cell - 2): the minimum-image threshold
-    double inv_req2;    // 1/r_eq^2
     float f_req, f_req2, f_req2_sel, f_kn, f_dc[3], f_gap[3], f_inv_vol, f_tanh2, f_dscale, f_apisig;
 };
 
@@ -105,7 +104,6 @@ static PC make_pc(const fipi_ctx* ctx) {
     c.inv_mu = 1.0 / c.mu;
     c.f_req = (float)c.r_eq;
     c.f_req2 = c.f_req * c.f_req;
-    c.inv_req2 = 1.0 / (c.r_eq * c.r_eq);
     // FP32 selection radius: a separation formed from cell-relative FP32
     // coordinates of up to 3 d_cell is off by less than 16 * 2^-24 d_cell per
     // axis (two conversions, the offset and its terms, two subtractions)
@@ -917,18 +915,6 @@ template <typename TA> __device__ __forceinline__ TA warp_total4(TA v0, TA v1, T
 __device__ __forceinline__ double min_image(double d, double thr, double L) {
     const long long m = __double_as_longlong(d) & 0x7fffffffffffffffll;
     return m > __double_as_longlong(thr) ? d - copysign(L, d) : d;
-}
-
-// r_eq / |d| from s = |d|^2 / r_eq^2 > 0: an FP32 estimate y and one
-// third-order (Halley) step y (1 + e/2 + 3 e^2/8), e = 1 - s y^2, whose
-// remainder is below e^3: rounding only.  s outside the FP32 range (or NaN)
-// takes the library's square root and division.
-__device__ __forceinline__ double inv_distance(double s) {
-    const long long b = __double_as_longlong(s);
-    if (b < 0x3990000000000000ll || b >= 0x4660000000000000ll) return 1.0 / sqrt(s);  // 2^-102, 2^103
-    const double y = (double)rsqrtf((float)s);
-    const double e = fma(-(s * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // Queues the staged candidates of home particle i (at h in the home frame)
@@ -2546,23 +2532,14 @@ __global__ void k_adj_stage(PC pc, int stage, const double* __restrict__ p, cons
 // i being F(d) with d = p_i - p_j for either id order (f_pp[it] += F,
 // f_pp[id] -= F, cluster.cpp:246-255), F(d) = (r_eq - |d|) ramp k_n d / |d|.
 // Coincident pairs (random separation in the reference) contribute nothing.
-// The terms of one pair, added to acc (lam_p[i]) and acc_kn (pkn[i]); d is
-// p_i - p_j by the minimum-image rule, li = lamF[i].  The k_n term
-// lamF[i] . (force on i) / k_n is F(d) . li / k_n.
+// A pair's terms, added to acc (lam_p[i]) and acc_kn (pkn[i]); d is p_i - p_j by
+// the minimum-image rule, li = lamF[i].
 __device__ __forceinline__ void pair_adj(const PC& pc, const double d[3], const double li[3],
                                          const double* __restrict__ lamF, int j, double rmp, double acc[3],
                                          double& acc_kn) {
     const int n = pc.n;
-    const double s = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0])) * pc.inv_req2;
-    if (!nonzero_bits(s)) return;
-    const double q = inv_distance(s);  // r_eq / |d|
-    const double g = q - 1.0;
-    if (!(g > 0.0)) return;
     const double dl[3] = {li[0] - lamF[j], li[1] - lamF[n + j], li[2] - lamF[2 * n + j]};
-    const double sc = rmp * pc.k_n, a = sc * g;
-    const double b = (sc * q) * (q * q * pc.inv_req2) * fma(d[2], dl[2], fma(d[1], dl[1], d[0] * dl[0]));
-    for (int e = 0; e < 3; ++e) acc[e] = fma(a, dl[e], fma(-b, d[e], acc[e]));
-    acc_kn = fma(g * rmp, fma(d[2], li[2], fma(d[1], li[1], d[0] * li[0])), acc_kn);
+    pair_adjoint(d, pc.r_eq, rmp, pc.k_n, dl, li, acc, acc_kn);
 }
 
 // One warp per home particle, FP32 selection (k_f_pp_warp).

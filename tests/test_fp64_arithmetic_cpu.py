@@ -148,3 +148,37 @@ int main() {
 
 def test_density_is_the_references(tmp_path):
     _run(tmp_path, DENSITY)
+
+
+# the adjoint's pair terms: the sums of the expressions with divisions, bit for bit,
+# from nearly touching centres to the contact range, and nothing outside it
+PAIR = r"""
+int main() {
+    long bad = 0;
+    for (int i = 0; i < 4000000; ++i) {
+        const double r_eq = fabs(draw(-4, 6)), rmp = (double)(1 + rng() % 100) / 100, k_n = fabs(draw(-6, 6));
+        double d[3] = {draw(-20, 0), draw(-20, 0), draw(-20, 0)}, dl[3], li[3];
+        const double far = r_eq * std::pow(2.0, -(double)(rng() % 4096) / 128 + 0.1) /
+                           std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        for (int e = 0; e < 3; ++e) { d[e] *= far; dl[e] = draw(-10, 3); li[e] = draw(-10, 3); }
+        if (i % 1000 == 0) d[0] = d[1] = d[2] = 0.0;
+        if (i % 1000 == 1) d[i % 3] = NAN;
+        double lam[3] = {draw(-5, 5), draw(-5, 5), draw(-5, 5)}, kn = draw(-5, 5);
+        double want[3] = {lam[0], lam[1], lam[2]}, want_kn = kn;
+        const double dn = std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        if (dn < r_eq && dn != 0.0) {
+            const double a = r_eq / dn - 1.0, b = r_eq / (dn * dn * dn) * (d[0] * dl[0] + d[1] * dl[1] + d[2] * dl[2]);
+            for (int e = 0; e < 3; ++e) want[e] += rmp * k_n * (a * dl[e] - b * d[e]);
+            want_kn += (r_eq - dn) * rmp / dn * (d[0] * li[0] + d[1] * li[1] + d[2] * li[2]);
+        }
+        pair_adjoint(d, r_eq, rmp, k_n, dl, li, lam, kn);
+        bad += lam[0] != want[0] || lam[1] != want[1] || lam[2] != want[2] || kn != want_kn;
+    }
+    std::printf("%ld\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def test_pair_adjoint_is_the_divisions(tmp_path):
+    _run(tmp_path, PAIR)
