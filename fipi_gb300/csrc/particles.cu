@@ -1508,12 +1508,13 @@ __device__ __forceinline__ void cell_and_frac(const PC& pc, double X, double Y, 
 // Spreading in ascending particle id without a sort.  Every record (particle
 // * 8 + corner) is pushed onto a linked list of its node (head, next; an
 // arbitrary order); then the record at the head of a list owns the node:
-// it brings the list into ascending order, sums it in that order (the order of
-// the reference's loop, cluster.cpp:368-406, so the sums are the same
-// whatever the order of the pushes) and leaves the head empty (-1) for the next
-// spread.  Two launches for what took a radix sort of the records in twelve:
-// FP64, 256 particles at 64^3 102 -> 25 us, 20,000 at 256^3 173 -> 63 (sums of
-// launches timed one by one).
+// the list is summed in ascending order (the order of the reference's loop,
+// cluster.cpp:368-406, so the sums are the same whatever the order of the
+// pushes) and its head left empty (-1) for the next spread.  Two launches for
+// what took a radix sort of the records in twelve.  FP64, sums of launches timed
+// one by one, sort -> lists: 256 particles at 64^3 93 -> 23 us, 20,000 at 256^3
+// 164 -> 52; the same in smaller and smaller clouds, 64 records a node 438 -> 246,
+// 256 633 -> 537, 1000 2205 -> 1280, all in one cell 18,600 -> 2,900.
 //
 // Records 8n of a push: node, and the list links.
 struct NodeLists {
@@ -1525,68 +1526,125 @@ __device__ __forceinline__ void push_record(const NodeLists& nl, int rec, unsign
     nl.nodes[rec] = node;
     nl.next[rec] = atomicExch(&nl.head[node], rec);
 }
-// Ascending order of the list from `h` (bottom-up merge sort on the links);
-// returns the new first record.
-__device__ __noinline__ int sort_links(int* next, int h) {
-    for (int width = 1;; width *= 2) {
-        int left = h, tail = -1, merges = 0;
-        h = -1;
-        while (left >= 0) {
-            ++merges;
-            int right = left, nl = 0, nr = width;
-            while (nl < width && right >= 0) {
-                right = next[right];
-                ++nl;
+// Sums of the lists at whose heads the threads' records are (one record s a
+// thread), in ascending record order: value(rec, v) gives the NA terms of a
+// record, store(node, a, sum) takes term a's sum.  Lists of up to kFewRecords
+// are brought into order in their thread's registers.  Longer ones (particles
+// gathered on a node) take the whole warp (a thread's merge sort of the links took
+// twice the sort's time at 128 records a node, ten times at 20,000): up to
+// kLongRecords are ranked in shared memory, beyond that the warp looks through
+// the nodes of all records, which are in order as they stand; the terms are
+// formed 32 at a time and added by one lane per term.  nrec records in all.
+constexpr int kFewRecords = 8, kLongRecords = 512, kSumThreads = 128;
+template <int NA, typename TA> struct LongLists {
+    int rec[kSumThreads / 32][kLongRecords], sorted[kSumThreads / 32][kLongRecords];
+    TA val[kSumThreads / 32][NA][32];
+};
+template <int NA, typename TA, class Value, class Store>
+__device__ __forceinline__ void sum_node_lists(const NodeLists& nl, int nrec, Value&& value, Store&& store) {
+    __shared__ LongLists<NA, TA> sh;
+    // Consecutive records go to different warps: the records at the heads are the ones
+    // pushed last, a few particles' (with a warp's records consecutive 2,000
+    // particles with 64 records a node took 143 us, one warp for eight lists).
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int s = lane * (int)gridDim.x * (kSumThreads / 32) + (int)blockIdx.x * (kSumThreads / 32) + w;
+    const unsigned node = s < nrec ? nl.nodes[s] : 0u;
+    const bool own = s < nrec && nl.head[node] == s;
+    int few[kFewRecords], m = 0;
+    if (own) {
+        for (int q = s; q >= 0 && m <= kFewRecords; q = nl.next[q]) {
+            if (m < kFewRecords) {
+                int at = m;  // insertion into the ascending prefix
+#pragma unroll
+                for (int k = kFewRecords - 1; k > 0; --k)
+                    if (k <= at && few[k - 1] > q) {
+                        few[k] = few[k - 1];
+                        at = k - 1;
+                    }
+#pragma unroll
+                for (int k = 0; k < kFewRecords; ++k)
+                    if (k == at) few[k] = q;
             }
-            while (nl > 0 || (nr > 0 && right >= 0)) {
-                int q;
-                if (nl > 0 && (nr == 0 || right < 0 || left < right)) {
-                    q = left;
-                    left = next[left];
-                    --nl;
-                } else {
-                    q = right;
-                    right = next[right];
-                    --nr;
+            ++m;
+        }
+        if (m <= kFewRecords) {
+            TA acc[NA] = {};
+#pragma unroll
+            for (int k = 0; k < kFewRecords; ++k)
+                if (k < m) {
+                    TA v[NA];
+                    value(few[k], v);
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) acc[a] += v[a];
                 }
-                if (tail < 0) h = q;
-                else next[tail] = q;
-                tail = q;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) store(node, a, acc[a]);
+            nl.head[node] = -1;
+        }
+    }
+    for (unsigned rest = __ballot_sync(0xffffffffu, own && m > kFewRecords); rest; rest &= rest - 1) {
+        const int l = __ffs(rest) - 1;
+        const int first = __shfl_sync(0xffffffffu, s, l);
+        const unsigned nd = __shfl_sync(0xffffffffu, node, l);
+        int *rec = sh.rec[w], *sorted = sh.sorted[w];
+        TA acc = TA(0);  // lane a < NA: the sum of term a
+        auto add = [&](int r, int count) {  // the records r of the first `count` lanes
+            TA v[NA];
+            if (lane < count) {
+                value(r, v);
+#pragma unroll
+                for (int a = 0; a < NA; ++a) sh.val[w][a][lane] = v[a];
             }
-            left = right;
-        }
-        if (tail >= 0) next[tail] = -1;
-        if (merges <= 1) return h;
-    }
-}
-// Calls add(record) for the records of the list owned by `rec` (which is at
-// its head) in ascending order and empties the list.
-template <class Add> __device__ __forceinline__ void owned_records(const NodeLists& nl, int rec, unsigned node, Add&& add) {
-    constexpr int kFew = 8;
-    int few[kFew], m = 0;
-    for (int q = rec; q >= 0; q = nl.next[q]) {
-        if (m < kFew) {
-            int at = m;  // insertion into the ascending prefix
+            __syncwarp();
+            if (lane < NA)
+                for (int k = 0; k < count; ++k) acc += sh.val[w][lane][k];
+            __syncwarp();
+        };
+        int c = 0;
+        for (int q = first; q >= 0 && c <= kLongRecords; q = nl.next[q], ++c)
+            if (lane == 0 && c < kLongRecords) rec[c] = q;
+        __syncwarp();
+        if (c <= kLongRecords) {
+            for (int e = lane; e < c; e += 32) {
+                const int q = rec[e];
+                int rank = 0;
+                for (int k = 0; k < c; ++k) rank += rec[k] < q;
+                sorted[rank] = q;
+            }
+            __syncwarp();
+            for (int e = 0; e < c; e += 32) add(e + lane < c ? sorted[e + lane] : 0, min(32, c - e));
+        } else {
+            int held = 0;  // matching records queued in rec, fewer than 32
+            for (int base = 0; base < nrec; base += 256) {
+                unsigned at[8];
 #pragma unroll
-            for (int k = kFew - 1; k > 0; --k)
-                if (k <= at && few[k - 1] > q) {
-                    few[k] = few[k - 1];
-                    at = k - 1;
+                for (int k = 0; k < 8; ++k) {
+                    const int r = base + 32 * k + lane;
+                    at[k] = r < nrec ? nl.nodes[r] : ~nd;
                 }
 #pragma unroll
-            for (int k = 0; k < kFew; ++k)
-                if (k == at) few[k] = q;
+                for (int k = 0; k < 8; ++k) {
+                    const unsigned hit = __ballot_sync(0xffffffffu, at[k] == nd);
+                    if (hit == 0) continue;
+                    if (at[k] == nd) rec[held + __popc(hit & ((1u << lane) - 1u))] = base + 32 * k + lane;
+                    held += __popc(hit);
+                    __syncwarp();
+                    if (held >= 32) {
+                        add(rec[lane], 32);
+                        held -= 32;
+                        const int left = lane < held ? rec[32 + lane] : 0;
+                        __syncwarp();
+                        if (lane < held) rec[lane] = left;
+                        __syncwarp();
+                    }
+                }
+            }
+            if (held > 0) add(lane < held ? rec[lane] : 0, held);
         }
-        ++m;
+        if (lane < NA) store(nd, lane, acc);
+        if (lane == 0) nl.head[nd] = -1;
+        __syncwarp();
     }
-    if (m <= kFew) {
-#pragma unroll
-        for (int k = 0; k < kFew; ++k)
-            if (k < m) add(few[k]);
-    } else {
-        for (int q = sort_links(nl.next, rec); q >= 0; q = nl.next[q]) add(q);
-    }
-    nl.head[node] = -1;
 }
 
 // Per particle: its 8 corner records, the force density f = (f_pp + f_ext)/dx
@@ -1637,21 +1695,17 @@ __device__ __forceinline__ TA corner_value(TA f, int c, TA o, TA pp, TA q) {
 }
 
 template <typename TF, typename TA>
-__global__ void k_spread_sum(int n, NodeLists nl, const TA* __restrict__ fw, TF* f0, TF* f1, TF* f2) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= 8 * n) return;
-    const unsigned node = nl.nodes[s];
-    if (nl.head[node] != s) return;
-    TA acc[3] = {TA(0), TA(0), TA(0)};
-    owned_records(nl, s, node, [&](int rec) {
-        const int i = rec >> 3, c = rec & 7;
-        const TA o = fw[3 * n + i], pp = fw[4 * n + i], qq = fw[5 * n + i];
+__global__ void __launch_bounds__(kSumThreads) k_spread_sum(int n, NodeLists nl, const TA* __restrict__ fw, TF* f0,
+                                                            TF* f1, TF* f2) {
+    sum_node_lists<3, TA>(
+        nl, 8 * n,
+        [&](int rec, TA* v) {
+            const int i = rec >> 3, c = rec & 7;
+            const TA o = fw[3 * n + i], pp = fw[4 * n + i], qq = fw[5 * n + i];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) acc[a] += corner_value<TA>(fw[a * n + i], c, o, pp, qq);
-    });
-    f0[node] = (TF)acc[0];
-    f1[node] = (TF)acc[1];
-    f2[node] = (TF)acc[2];
+            for (int a = 0; a < 3; ++a) v[a] = corner_value<TA>(fw[a * n + i], c, o, pp, qq);
+        },
+        [&](unsigned node, int a, TA sum) { (a == 0 ? f0 : a == 1 ? f1 : f2)[node] = (TF)sum; });
 }
 
 // ------------------------------------------------------------ orchestration
@@ -1664,7 +1718,7 @@ static void spread_t(fipi_ctx* ctx, const double* p, const double* f_pp, T* cons
     const PC pc = make_pc(ctx);
     const int n = b.n;
     { LaunchScope ls_(ctx, "spread records", 0.0); k_spread_push<T, T><<<(n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, p, f_pp, nl, (T*)b.sp_fw, clear_prev ? 1 : 0, f3[0], f3[1], f3[2]); }
-    { LaunchScope ls_(ctx, "spread sums", 0.0); k_spread_sum<T, T><<<(8 * n + 127) / 128, 128, 0, ctx->stream>>>(n, nl, (const T*)b.sp_fw, f3[0], f3[1], f3[2]); }
+    { LaunchScope ls_(ctx, "spread sums", 0.0); k_spread_sum<T, T><<<(8 * n + kSumThreads - 1) / kSumThreads, kSumThreads, 0, ctx->stream>>>(n, nl, (const T*)b.sp_fw, f3[0], f3[1], f3[2]); }
 }
 
 // Mixed-form spreading of the step: the 8 FP32 corner contributions of each
@@ -2640,19 +2694,17 @@ __global__ void k_adj_push(PC pc, const double* __restrict__ p0, const double* _
 }
 
 // part[q][node] = sum of w_c lam_q in ascending record order.
-__global__ void k_adj_sum(NodeLists nl, int ne, const double* __restrict__ rw, double* part, size_t V) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= 8 * ne) return;
-    const unsigned node = nl.nodes[s];
-    if (nl.head[node] != s) return;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    owned_records(nl, s, node, [&](int rec) {
-        const int e = rec >> 3, c = rec & 7;
-        const double o = rw[e], pp = rw[ne + e], qq = rw[2 * ne + e];
+__global__ void __launch_bounds__(kSumThreads) k_adj_sum(NodeLists nl, int ne, const double* __restrict__ rw,
+                                                         double* part, size_t V) {
+    sum_node_lists<4, double>(
+        nl, 8 * ne,
+        [&](int rec, double* v) {
+            const int e = rec >> 3, c = rec & 7;
+            const double o = rw[e], pp = rw[ne + e], qq = rw[2 * ne + e];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += corner_value<double>(rw[(3 + k) * ne + e], c, o, pp, qq);
-    });
-    for (int k = 0; k < 4; ++k) part[k * V + node] = acc[k];
+            for (int k = 0; k < 4; ++k) v[k] = corner_value<double>(rw[(3 + k) * ne + e], c, o, pp, qq);
+        },
+        [&](unsigned node, int a, double sum) { part[a * V + node] = sum; });
 }
 
 // Adjoint of the spreading of f_pp^n at p^n given lamF (3 real fields).
@@ -2760,7 +2812,7 @@ fipi_status particles_adjoint(fipi_ctx* ctx) {
     const NodeLists nl{b.sp_head, a.rnext, a.rnode};
     if (!a.part_valid) FIPI_CUDA(ctx, cudaMemsetAsync(a.part, 0, sizeof(double) * 4 * V, ctx->stream));
     { LaunchScope ls_(ctx, "adjoint: records", 0.0); k_adj_push<<<(2 * n + kPT - 1) / kPT, kPT, 0, ctx->stream>>>(pc, a.in.p0, a.p1, a.lamloc, nl, a.rw, a.part_valid ? 1 : 0, a.part, V); }
-    { LaunchScope ls_(ctx, "adjoint: record sums", 0.0); k_adj_sum<<<(16 * n + 127) / 128, 128, 0, ctx->stream>>>(nl, 2 * n, a.rw, a.part, V); }
+    { LaunchScope ls_(ctx, "adjoint: record sums", 0.0); k_adj_sum<<<(16 * n + kSumThreads - 1) / kSumThreads, kSumThreads, 0, ctx->stream>>>(nl, 2 * n, a.rw, a.part, V); }
     a.part_valid = true;
     FIPI_CUDA(ctx, cudaGetLastError());
     return FIPI_OK;
