@@ -64,6 +64,7 @@ struct ParticleBufs {
     // spreading: node lists of the FP64 form (particles.cu, NodeLists)
     int* sp_head = nullptr;           // V, -1 between spreads
     int* sp_next = nullptr;           // 8n
+    unsigned* sp_call = nullptr;      // 8n nodes of a fine-grained call
     unsigned* sp_prev = nullptr;      // 8n nodes written by the previous spread
     // mixed form: per node 32 bytes, the three fixed-point spread sums and,
     // in the low half of the fourth word, the FP32 sum of |contribution|
