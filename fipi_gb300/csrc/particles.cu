@@ -321,9 +321,8 @@ __global__ void k_cells_count(PC pc, const double* __restrict__ p, unsigned* key
     }
 }
 
-// Exclusive scan of ncells counts into off[0..ncells] (one block); the counts
-// are zero again afterwards, ready for the next list.
-__global__ void k_cells_scan(int* __restrict__ cnt, int ncells, int* off) {
+// Exclusive scan of ncells counts into off[0..ncells] (one block).
+__global__ void k_cells_scan(const int* __restrict__ cnt, int ncells, int* off) {
     __shared__ int part[1024];
     const int t = threadIdx.x;
     const int chunk = (ncells + 1023) / 1024;
@@ -342,7 +341,6 @@ __global__ void k_cells_scan(int* __restrict__ cnt, int ncells, int* off) {
     for (int i = b; i < e; ++i) {
         off[i] = run;
         run += cnt[i];
-        cnt[i] = 0;
     }
     if (t == 1023) off[ncells] = part[1023];
 }
@@ -372,8 +370,10 @@ __device__ __forceinline__ void sorted_pos(const PC& pc, const double* __restric
 }
 
 // One warp per cell: rank of each id among the cell's ids.  With spos the
-// sorted positions of the contact forces are written as well.
-__global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __restrict__ off, int ncells,
+// sorted positions of the contact forces are written as well.  The cell's count is
+// zero again afterwards, ready for the next list (zeroed by the scan, one
+// block with a run of cells per thread, it cost 705 -> 1165 us for 614,000 cells).
+__global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __restrict__ off, int* cnt, int ncells,
                               const unsigned* __restrict__ tmp, unsigned* ids, unsigned* skeys,
                               unsigned long long* ymax, int* it_mark, float4* spos) {
     const int cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -384,6 +384,7 @@ __global__ void k_cells_order(PC pc, const double* __restrict__ p, const int* __
         ymax[1] = ~0ull;
     }
     if (cell >= ncells) return;
+    if (lane == 0) cnt[cell] = 0;
     const int beg = off[cell], end = off[cell + 1];
     const int cx = cell % pc.nc[0], cy = (cell / pc.nc[0]) % pc.nc[1], cz = cell / (pc.nc[0] * pc.nc[1]);
     for (int e = beg + lane; e < end; e += 32) {
@@ -507,7 +508,7 @@ static bool build_cells(fipi_ctx* ctx, const double* p_dev, bool want_it_mark = 
     }
     { LaunchScope ls_(ctx, "cell offsets", 0.0); k_cells_scan<<<1, 1024, 0, ctx->stream>>>(b.cell_cnt, b.ncells, b.cell_off); }
     { LaunchScope ls_(ctx, "cell placement", 0.0); k_cells_place<<<nb, kPT, 0, ctx->stream>>>(pc, p_dev, b.keys_alt, b.ids_alt, b.cell_off, b.keys, ym); }
-    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos); }
+    { LaunchScope ls_(ctx, "cell order", 0.0); k_cells_order<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, p_dev, b.cell_off, b.cell_cnt, b.ncells, b.keys, b.ids, b.keys_alt, ym, b.it_mark, spos); }
     std::swap(b.keys, b.keys_alt);  // sorted keys now in keys
     return want_it_mark;
 }
