@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(32 * kFppRows) k_f_pp_fast(PC pc, const float4
     const int cw = (ci + (lane % 3) - 1 + pc.nc[0]) % pc.nc[0] + rowbase;
     const int r6 = lane < 6 ? off[cw + (lane >= 3 ? 1 : 0)] : 0;
     const int beg = off[cell], end = off[cell + 1];
+    if (beg == end) return;  // the whole block (1000 particles in 614,000 cells 1440 -> 1030 us)
     int qb[3], qe[3], held[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -949,17 +950,12 @@ __device__ __forceinline__ void fpp_select(const PC& pc, const FppShared& sh, in
     }
 }
 
-// The block's home particles, one per warp and round: body(i)'s pair functor
-// for every selected candidate, then done(i, ...).  blockIdx.x = cell,
-// blockIdx.y of gridDim.y shares of its particles.
+// One home cell.
 template <class Home>
-__device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict__ spos, const int* __restrict__ off,
-                                          Home&& home) {
-    __shared__ FppShared sh;
-    const int cell = blockIdx.x;
-    const int hb = off[cell], nh = off[cell + 1] - hb;
-    if ((int)blockIdx.y * kFppWarps >= nh) return;  // the whole block
+__device__ __forceinline__ void fpp_home_cell(const PC& pc, const float4* __restrict__ spos,
+                                              const int* __restrict__ off, FppShared& sh, int cell, Home&& home) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int hb = off[cell], nh = off[cell + 1] - hb;
     fpp_cells(pc, cell, off, sh);
     __syncthreads();
     const int total = sh.pre[27];
@@ -985,6 +981,24 @@ __device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict
     }
 }
 
+// The home particles of the block's cells, one per warp and round: body(i)'s pair
+// functor for every selected candidate, then done(i, ...).  blockIdx.x: `cells`
+// consecutive cells (at most 32), blockIdx.y of gridDim.y shares of their particles.
+template <class Home>
+__device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict__ spos, const int* __restrict__ off,
+                                          int cells, Home&& home) {
+    __shared__ FppShared sh;
+    const int lane = threadIdx.x & 31;
+    const int mine = blockIdx.x * cells + lane;
+    int nh = 0;
+    if (lane < cells && mine < pc.nc[0] * pc.nc[1] * pc.nc[2]) nh = off[mine + 1] - off[mine];
+    // the same in every warp
+    for (unsigned rest = __ballot_sync(0xffffffffu, (int)blockIdx.y * kFppWarps < nh); rest; rest &= rest - 1) {
+        fpp_home_cell(pc, spos, off, sh, blockIdx.x * cells + __ffs(rest) - 1, home);
+        __syncthreads();  // the next cell's candidates take the place of this one's
+    }
+}
+
 // TA: the arithmetic the forces are formed and summed in (k_f_pp's): double in
 // the FP64 form, each pair's force being the reference's bit for bit (a square
 // root, a reciprocal and products in its order: 173 us at 256^3 where a
@@ -993,20 +1007,20 @@ __device__ __forceinline__ void fpp_block(const PC& pc, const float4* __restrict
 // one after the other in the reference's pair order, so that the mixed form's
 // forces are k_f_pp<float>'s bit for bit.
 template <typename TA>
-__global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const double* __restrict__ p,
+__global__ void __launch_bounds__(32 * kFppWarps, 7) k_f_pp_warp(PC pc, const double* __restrict__ p,
                                                               const float4* __restrict__ spos,
                                                               const int* __restrict__ off,
                                                               const double* __restrict__ rmp_p,
                                                               const double* __restrict__ f_pi,
                                                               const int* __restrict__ it_mark, double* f_pp,
-                                                              double* tau_part) {
+                                                              double* tau_part, int cells) {
     const int n = pc.n;
     bool mark = false;
     if (f_pi != nullptr) {
         const int m = *it_mark;
         mark = m >= 0 && any_force(f_pi, n, m);
     }
-    fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
+    fpp_block(pc, spos, off, cells, [&](float4 h, bool on, int lane, auto&& walk) {
         const int i = __float_as_int(h.w);
         const bool tau_on = mark && any_force(f_pi, n, i);
         const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
@@ -1073,13 +1087,21 @@ __global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_warp(PC pc, const doubl
     });
 }
 
-// Blocks per home cell: enough that every SM has several.
-static dim3 fpp_grid(const fipi_ctx* ctx) {
+// Blocks per home cell: enough that every SM has several.  Cells per block: where
+// most cells are empty, as many as hold about one particle, and no fewer blocks
+// than eight an SM (1000 particles in 614,000 cells: 20 us; a block for every
+// cell took 315, k_f_pp 250).
+struct FppGrid {
+    dim3 blocks;
+    int cells;
+};
+static FppGrid fpp_grid(const fipi_ctx* ctx) {
     const ParticleBufs& b = ctx->pb;
+    const int cells = std::max(1, std::min(std::min(b.ncells / std::max(b.n, 1), b.ncells / (8 * ctx->num_sms)), 32));
     const int per_cell = b.n / b.ncells + 1;
     int shares = (4 * ctx->num_sms + b.ncells - 1) / b.ncells;
     shares = std::min(shares, (per_cell + kFppWarps - 1) / kFppWarps);
-    return dim3(b.ncells, std::max(1, shares));
+    return {dim3((b.ncells + cells - 1) / cells, std::max(1, shares)), cells};
 }
 
 // it_mark of cluster::sorting (cluster.cpp:128-138): the first index of
@@ -1891,10 +1913,12 @@ static void f_pp_launch(fipi_ctx* ctx, const double* p, const double* rmp, const
         if (path == FppPath::fast)
             k_f_pp_fast<<<b.ncells, 32 * kFppRows, 0, ctx->stream>>>(pc, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr,
                                                                      b.it_mark, f_pp, tau ? b.tau_part : nullptr);
-        else
-            k_f_pp_warp<TA><<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(
+        else {
+            const FppGrid fg = fpp_grid(ctx);
+            k_f_pp_warp<TA><<<fg.blocks, 32 * kFppWarps, 0, ctx->stream>>>(
                 pc, p, b.spos, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark, f_pp,
-                tau ? b.tau_part : nullptr);
+                tau ? b.tau_part : nullptr, fg.cells);
+        }
     } else {
         const int blocks = (b.ncells * 32 + 255) / 256;
         { LaunchScope ls_(ctx, "contact forces (warp per cell)", 0.0); k_f_pp<TA, 0><<<blocks, 256, 0, ctx->stream>>>(pc, p, b.ids, b.cell_off, rmp, tau ? f_pi : nullptr, b.it_mark,
@@ -2607,15 +2631,15 @@ __device__ __forceinline__ void pair_adj(const PC& pc, const double d[3], const 
 }
 
 // One warp per home particle, FP32 selection (k_f_pp_warp).
-__global__ void __launch_bounds__(32 * kFppWarps) k_f_pp_adj_warp(PC pc, const double* __restrict__ p,
+__global__ void __launch_bounds__(32 * kFppWarps, 7) k_f_pp_adj_warp(PC pc, const double* __restrict__ p,
                                                                   const float4* __restrict__ spos,
                                                                   const int* __restrict__ off,
                                                                   const double* __restrict__ rmp_p,
                                                                   const double* __restrict__ lamF, double* lam_p,
-                                                                  double* pkn) {
+                                                                  double* pkn, int cells) {
     const int n = pc.n;
     const double rmp = *rmp_p;
-    fpp_block(pc, spos, off, [&](float4 h, bool on, int lane, auto&& walk) {
+    fpp_block(pc, spos, off, cells, [&](float4 h, bool on, int lane, auto&& walk) {
         const int i = __float_as_int(h.w);
         const double xi = p[i], yi = p[n + i], zi = p[2 * n + i];
         const double li[3] = {lamF[i], lamF[n + i], lamF[2 * n + i]};
@@ -2793,9 +2817,10 @@ fipi_status particles_adjoint(fipi_ctx* ctx) {
     float4* spos = f_pp_path(ctx, false) != FppPath::cell ? b.spos : nullptr;
     auto contact_adj = [&](const double* q, const double* lamF, double* lam_p) {
         LaunchScope ls_(ctx, "adjoint: contact forces", 0.0);
+        const FppGrid fg = fpp_grid(ctx);
         if (spos)
-            k_f_pp_adj_warp<<<fpp_grid(ctx), 32 * kFppWarps, 0, ctx->stream>>>(pc, q, spos, b.cell_off, a.rmp, lamF,
-                                                                               lam_p, a.pp_kn);
+            k_f_pp_adj_warp<<<fg.blocks, 32 * kFppWarps, 0, ctx->stream>>>(pc, q, spos, b.cell_off, a.rmp, lamF, lam_p,
+                                                                           a.pp_kn, fg.cells);
         else
             k_f_pp_adj<<<(b.ncells * 32 + 255) / 256, 256, 0, ctx->stream>>>(pc, q, b.ids, b.cell_off, a.rmp, lamF,
                                                                              lam_p, a.pp_kn);
