@@ -16,12 +16,9 @@ namespace fipi {
 // Device buffers of one precision form.  T = float (mixed) or double.
 struct FieldBufs {
     void* tables = nullptr;  // the tables below
-    void* twx = nullptr;  // exp(-2 pi i q / nx), q < nx     (cplx<T>)
+    void* twx = nullptr;  // exp(-2 pi i q / nx), q < nx     (tw_t<T>)
     void* twy = nullptr;  // exp(-2 pi i q / ny)
     void* twz = nullptr;  // exp(-2 pi i q / nz)
-    void* fwx = nullptr;  // the twiddles as block fixed-point factors (FP64 form, fx64.cuh)
-    void* fwy = nullptr;
-    void* fwz = nullptr;
     void* kx = nullptr;   // wave numbers (T): kx[0..M], ky[0..ny), kz[0..nz)
     void* ky = nullptr;
     void* kz = nullptr;

@@ -601,7 +601,7 @@ template <typename T> static fipi_status alloc_fields_t(fipi_ctx* ctx) {
         at.push_back({dst, o});
     };
     std::vector<std::pair<long double, long double>> cs;  // cos, sin of 2 pi q / cs.size()
-    auto twiddles = [&](int n, void** tw, void** fw) {
+    auto twiddles = [&](int n, void** tw) {
         if ((int)cs.size() != n) {
             cs.resize(n);
             const long double two_pi = 6.283185307179586476925286766559005768L;
@@ -610,25 +610,22 @@ template <typename T> static fipi_status alloc_fields_t(fipi_ctx* ctx) {
                 cs[q] = {cosl(a), sinl(a)};
             }
         }
-        std::vector<C> t(n);
+        std::vector<tw_t<T>> t(n);
         for (int q = 0; q < n; ++q) {
-            t[q].x = (T)cs[q].first;
-            t[q].y = (T)(-cs[q].second);
-        }
-        put(tw, t.data(), sizeof(C) * n);
-        if constexpr (sizeof(T) == sizeof(double)) {  // block fixed-point factors (fx64.cuh)
-            std::vector<longlong2> f(n);
-            const long double one = 4611686018427387904.0L;
-            for (int q = 0; q < n; ++q) {
-                f[q].x = fx_pack(llrintl(cs[q].first * one));
-                f[q].y = fx_pack(llrintl(-cs[q].second * one));
+            if constexpr (sizeof(T) == sizeof(double)) {  // block fixed-point factors (fx64.cuh)
+                const long double one = 4611686018427387904.0L;
+                t[q].x = fx_pack(llrintl(cs[q].first * one));
+                t[q].y = fx_pack(llrintl(-cs[q].second * one));
+            } else {
+                t[q].x = (T)cs[q].first;
+                t[q].y = (T)(-cs[q].second);
             }
-            put(fw, f.data(), sizeof(longlong2) * n);
         }
+        put(tw, t.data(), sizeof(tw_t<T>) * n);
     };
-    twiddles(g.nx, &b.twx, &b.fwx);
-    twiddles(g.ny, &b.twy, &b.fwy);
-    twiddles(g.nz, &b.twz, &b.fwz);
+    twiddles(g.nx, &b.twx);
+    twiddles(g.ny, &b.twy);
+    twiddles(g.nz, &b.twz);
     // field.cpp:100-121: i*2.0*pi/L for i <= N/2 else (i - N)*2.0*pi/L
     const fipi_params& P = ctx->P;
     auto waves = [&](void** dst, int n, int count, double L) {

@@ -466,7 +466,7 @@ __device__ __forceinline__ void fx_r2c_row(double2* s, const Idx& idx, int row, 
 // live in shared memory with one pad slot per 16 (pitch odd, so the
 // transposed column accesses are conflict-free); X_M sits at index M.
 // Blocks per SM the register budget is set for: FP32 4 (3 with four
-// fields), FP64 3 (2).  512-thread blocks measured slower.
+// fields), FP64 by rows and fields (XMinBlocks).  512-thread blocks measured slower.
 // Rows per X-pass tile: 16 FP32 rows (8 FP64) keep 128-byte runs along y;
 // FP32 rows of 512 points take 8 so that the tile of four fields fits
 // three blocks per SM.
@@ -885,8 +885,7 @@ template <typename T> struct F {
     // the transforms' twiddle tables along x, y, z
     static const tw_t<T>* tw(const fipi_ctx* ctx, int axis) {
         const FieldBufs& b = ctx->fb;
-        constexpr bool fx = sizeof(T) == sizeof(double);
-        return (const tw_t<T>*)(axis == 0 ? (fx ? b.fwx : b.twx) : axis == 1 ? (fx ? b.fwy : b.twy) : (fx ? b.fwz : b.twz));
+        return (const tw_t<T>*)(axis == 0 ? b.twx : axis == 1 ? b.twy : b.twz);
     }
     static KTabs<T> ktabs(fipi_ctx* ctx) {
         return KTabs<T>{(const T*)ctx->fb.kx, (const T*)ctx->fb.ky, (const T*)ctx->fb.kz};
