@@ -215,8 +215,9 @@ template <typename T> struct OpForce {
 // over c_hat^{n-1} at the same index.
 //
 // The state arrays it reads and writes are not needed again before L2 has
-// turned over: streaming accesses in the FP64 form (450 -> 425 us at 256^3; the
-// mixed form's measured 111 -> 112 us, 1028 -> 1040 at 512^3, and are plain).
+// turned over: streaming accesses in the FP64 form (450 -> 425 us at 256^3; 475
+// with the quotients of the division; the mixed form's measured 111 -> 112 us,
+// 1028 -> 1040 at 512^3, and are plain).
 //
 // FP64 form: the reference's histories and evaluation order, with the
 // quotients of its divisions:

@@ -23,8 +23,9 @@
 // directions) against extended precision: 0.2 to 0.95 of the FP64 codelets'
 // (uniform noise 2.7e-16 -> 0.9e-16; offset noise, inverse, 512-point rows
 // 1.75e-16 -> 1.3e-16; with the growth bound alone 6.8e-16).
-// Measured at 256^3: three-field Y pass 1207 -> 326 us, force pass 4250 -> 1107,
-// projection round trip 4510 -> 2550.
+// Measured at 256^3: three-field Y pass 1207 -> 276 us, force pass 4250 -> 1001,
+// projection round trip 4510 -> 1209 (with the warp-owned rows and columns and the
+// quotients of fp64.cuh).
 //
 // Rows with an infinity or a NaN (E = 0x7ff) come out as NaN throughout.
 // Rows below 2^-959 are scaled up by 2^200 first, so subnormal inputs

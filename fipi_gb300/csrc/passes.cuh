@@ -495,8 +495,8 @@ template <typename T, int NF, int NT> struct XMinBlocks {
 // fields' rows (32 x 256 x 128: c, f pass 166 us with 256 threads, most of them
 // idle, 35 with 32).  The
 // register budget follows what the tile leaves room for.  At 256^3 against 256
-// threads with block-wide rounds: c, f 407 -> 242 us, conv 640 -> 505, force
-// 1107 -> 955.
+// threads with block-wide rounds: c, f 407 -> 242 us, conv 640 -> 521, force
+// 1107 -> 1001.
 template <int M, int NF> constexpr int x_fx_threads =
     M >= 32 ? x_rows_of(8, M) * FftPlan<M, 8>::Tn : (NF * x_rows_of(8, M) * FftPlan<M, 8>::Tn + 31) / 32 * 32;
 template <int NF, int NT> struct XMinBlocks<double, NF, NT> {
